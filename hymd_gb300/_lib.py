@@ -97,7 +97,7 @@ class ScrArgs(ctypes.Structure):
 
 class Kick(ctypes.Structure):
     """HpfKick of include/hpf_gb300.h."""
-    _fields_ = [("v", P), ("prev", P * 4), ("n_prev", I), ("pad", I), ("mass", D),
+    _fields_ = [("v", P), ("prev", P * 4), ("n_prev", I), ("defer", I), ("mass", D),
                 ("dt_outer", D), ("thermo", ctypes.POINTER(CsvrArgs)), ("group", P),
                 ("randoms", P), ("counter", P), ("state", P), ("ws", P), ("d_err", P)]
 
@@ -109,6 +109,7 @@ _SIGNATURES.update({
     "hpf_field_pic_step": [P, P, P, I64, ctypes.POINTER(D), P, P, P, P, P, I64, D, P, P,
                            ctypes.POINTER(Kick), I, P],
     "hpf_csvr_scale": [P, P, I64, P, I, P],
+    "hpf_csvr_apply": [P, P, I64, ctypes.POINTER(CsvrArgs), P, P, P, P, P, P],
     "hpf_field_step_profile": [P, P, P, I64, ctypes.POINTER(D), P, P, P, ctypes.POINTER(Kick), P,
                                ctypes.POINTER(ctypes.c_float)],
     "hpf_csvr": [P, P, I64, ctypes.POINTER(P), I, D, ctypes.POINTER(CsvrArgs), P, P, P, P, P, P],

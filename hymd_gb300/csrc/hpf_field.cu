@@ -25,17 +25,7 @@
 
 namespace {
 
-constexpr int kThreads = 256;
-
-// Blocks of the readout with the CSVR sums (a grid reduction): two per SM,
-// or up to four once each thread would otherwise handle more than three
-// beads.  Measured on GB300: 162k beads ran fastest on 304 blocks, 500k
-// beads on 608 (1.8 % faster than 304; 1024 blocks was slower than 608).
-inline int readout_grid(int64_t n) {
-    const int g = reduce_grid(n, kThreads);
-    const int64_t per3 = (n + 3 * kThreads - 1) / (3 * kThreads);
-    return per3 > g ? (int)std::min<int64_t>(per3, 2 * HPF_REDUCE_GRID) : g;
-}
+constexpr int kThreads = kReadoutThreads;
 
 struct TypeScale {
     float s[HPF_MAX_TYPES + 1];
@@ -271,7 +261,8 @@ __global__ void k_kspace_sums(const float2* __restrict__ phi_f, const float2* __
 }
 
 // ---------------------------------------------------------------- readout ---
-// Kick fused into the readout (MODE 1), plus CSVR velocity sums (MODE 2).
+// Kick fused into the readout (MODE 1), plus CSVR velocity sums and factors
+// (MODE 2), or the sums' block partials alone (MODE 3, for hpf_csvr_apply).
 struct KickDev {
     float* v;
     const float* prev[4];
@@ -372,7 +363,7 @@ __global__ void k_readout(const float* __restrict__ fm, const float* __restrict_
                 kd.v[3 * i + d] = x;
                 w[d] = x;
             }
-            if (MODE == 2) {
+            if (MODE >= 2) {
                 const int g = kd.group ? kd.group[i] : 0;
                 if (g == 0 || g == 1) {
                     acc[4 * g + 0] += w[0];
@@ -388,6 +379,7 @@ __global__ void k_readout(const float* __restrict__ fm, const float* __restrict_
         if (grid_reduce_store_f<8, kThreads>(acc, ws_partials(kd.ws), ws_ticket(kd.ws), kd.ws))
             csvr_update(kd.a, kd.ws, kd.randoms, kd.counter, kd.state, err);
     }
+    if (MODE == 3) block_partials_f<8, kThreads>(acc, ws_partials(kd.ws), gridDim.x);
 }
 
 // ------------------------------------------------------------------- PIC ---
@@ -840,12 +832,12 @@ int launch_readout(hpf_ctx* c, const float* fm, const float* pos, const int32_t*
             kd.counter = kick->counter;
             kd.state = kick->state;
             kd.ws = kick->ws;
-            mode = 2;
+            mode = kick->defer ? 3 : 2;
         }
     }
     if ((pos_w != nullptr) != (scale != nullptr) || (pos_w && mode == 1)) return HPF_ERR_ARG;
-    int* err = mode == 2 && kick->d_err ? kick->d_err : c->d_err;
-    const int grid = mode == 2 ? readout_grid(n) : grid_for(n, kThreads);
+    int* err = mode >= 2 && kick->d_err ? kick->d_err : c->d_err;
+    const int grid = mode >= 2 ? kick_readout_grid(n, kThreads) : grid_for(n, kThreads);
     const int32_t* no_idx = nullptr;
     const int64_t n_total = 0;
     cudaError_t e;
@@ -857,6 +849,12 @@ int launch_readout(hpf_ctx* c, const float* fm, const float* pos, const int32_t*
                        c->d_box, force, err, kd, no_idx, n_total, pos_w, scale);
     else if (mode == 1)
         e = launch_pdl(k_readout<1>, grid, kThreads, 0, st, fm, pos, types, charges, n, T, c->M,
+                       c->d_box, force, err, kd, no_idx, n_total, pos_w, scale);
+    else if (mode == 3 && pos_w)
+        e = launch_pdl(k_readout<3, true>, grid, kThreads, 0, st, fm, pos, types, charges, n, T,
+                       c->M, c->d_box, force, err, kd, no_idx, n_total, pos_w, scale);
+    else if (mode == 3)
+        e = launch_pdl(k_readout<3>, grid, kThreads, 0, st, fm, pos, types, charges, n, T, c->M,
                        c->d_box, force, err, kd, no_idx, n_total, pos_w, scale);
     else if (pos_w)
         e = launch_pdl(k_readout<2, true>, grid, kThreads, 0, st, fm, pos, types, charges, n, T,

@@ -156,6 +156,20 @@ static inline int reduce_grid(int64_t work, int threads) {
     return (int)b;
 }
 
+// Blocks of the readout with the kick and the CSVR velocity sums, by bead
+// count, and with deferred sums the partial slots per value that it leaves
+// (hpf_csvr_apply sums as many): two per SM, or up to four once a thread would
+// otherwise handle more than three beads.  Measured on GB300 with deferred
+// sums, whole step: 162k beads 99.1 us on 304 blocks, 101.6 on 608, 102.5 on
+// one bead per thread; 500k beads 278.7 on 304, 276.4 on 608, 280.7 on 1024.
+static inline int kick_readout_grid(int64_t n, int threads) {
+    const int g = reduce_grid(n, threads);
+    const int64_t per3 = (n + 3 * threads - 1) / (3 * threads);
+    if (per3 <= g) return g;
+    return (int)(per3 > 2 * HPF_REDUCE_GRID ? 2 * HPF_REDUCE_GRID : per3);
+}
+constexpr int kReadoutThreads = 256;
+
 // Derived box quantities, shared by the host setter and the device barostat.
 __host__ __device__ inline void fill_box_state(BoxState& s, double L0, double L1, double L2,
                                                const int n[3]) {
@@ -230,66 +244,114 @@ __device__ __forceinline__ void fill_box_state_dev(BoxState& s, float L0, float 
 // reference's check_thermostat_coupling_groups), so the group sums cover the
 // whole system.  alpha^2 is formed in FP32, as the O(1) factor has no
 // cancellation; K and the composed transforms are FP64.
-__device__ __forceinline__ void csvr_update(const HpfCsvrArgs& a, const double* ws,
-                                            const double* randoms, int* counter, double* state,
-                                            int* err) {
-    const int s = *counter;
-    const bool ok = s >= 0 && s < a.n_steps;
-    if (!ok) hpf_flag(err, HPF_ERR_INDEX);
-    const bool act = !(a.every > 1 && (s + 1) % a.every != 0);
+//
+// In three parts, so that a kernel whose every block needs the factors can
+// load the inputs that do not depend on the sums early, and only one block
+// stores the results: csvr_load, csvr_factors, csvr_store.
+struct CsvrIn {
+    int s;         // step = row of the random table
+    bool ok, act;  // row in the table; a step on which the thermostat acts
+    double iN[2];  // 1 / particles of each group
+    float R[2], S[2];
+};
+struct CsvrOut {
+    double A[2], B[2][3];  // v_final = A_h v + B_h
+    double work[2];        // K (alpha^2 - 1) of each group
+};
+
+__device__ __forceinline__ CsvrIn csvr_load(const HpfCsvrArgs& a, const double* randoms,
+                                            const int* counter, int* err) {
+    CsvrIn in;
+    in.s = *counter;
+    in.ok = in.s >= 0 && in.s < a.n_steps;
+    if (!in.ok) hpf_flag(err, HPF_ERR_INDEX);
+    in.act = !(a.every > 1 && (in.s + 1) % a.every != 0);
     const int ng = a.n_groups < 1 ? 1 : (a.n_groups > 2 ? 2 : a.n_groups);
-    double A[2] = {1.0, 1.0};
-    double B[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-    for (int g = 0; act && g < ng; ++g) {
+    for (int g = 0; g < 2; ++g) {
+        if (g >= ng) break;
+        const double* row = randoms + (int64_t)in.s * a.stride + a.offset + 2 * g;
+        in.iN[g] = 1.0 / a.count[g];
+        in.R[g] = in.ok ? (float)row[0] : 0.0f;
+        in.S[g] = in.ok ? (float)row[1] : 3.0f * (float)a.count[g] - 1.0f;
+    }
+    return in;
+}
+
+__device__ __forceinline__ CsvrOut csvr_factors(const HpfCsvrArgs& a, const CsvrIn& in,
+                                                const double* ws) {
+    const int ng = a.n_groups < 1 ? 1 : (a.n_groups > 2 ? 2 : a.n_groups);
+    CsvrOut o;
+    for (int h = 0; h < 2; ++h) {
+        o.A[h] = 1.0;
+        o.work[h] = 0.0;
+        for (int d = 0; d < 3; ++d) o.B[h][d] = 0.0;
+    }
+    for (int g = 0; g < 2; ++g) {
+        if (!in.act || g >= ng) break;
         const double N = a.count[g];
         const bool com = a.remove_com && N > 1.0;
         double cnow[3] = {0.0, 0.0, 0.0};
         double K;
         if (com) {
-            const double iN = 1.0 / N;
+            const double iN = in.iN[g];
             double c2 = 0.0;
             for (int d = 0; d < 3; ++d) {
                 const double c0 = ws[4 * g + d] * iN;
                 c2 += c0 * c0;
-                cnow[d] = A[g] * c0 + B[g][d];
+                cnow[d] = o.A[g] * c0 + o.B[g][d];
             }
-            K = 0.5 * a.mass * A[g] * A[g] * (ws[4 * g + 3] - N * c2);
+            K = 0.5 * a.mass * o.A[g] * o.A[g] * (ws[4 * g + 3] - N * c2);
         } else {
             K = 0.0;
-            for (int h = 0; h < ng; ++h) {
+            for (int h = 0; h < 2; ++h) {
+                if (h >= ng) break;
                 double bs = 0.0, bb = 0.0;
                 for (int d = 0; d < 3; ++d) {
-                    bs += B[h][d] * ws[4 * h + d];
-                    bb += B[h][d] * B[h][d];
+                    bs += o.B[h][d] * ws[4 * h + d];
+                    bb += o.B[h][d] * o.B[h][d];
                 }
-                K += A[h] * A[h] * ws[4 * h + 3] + 2.0 * A[h] * bs + a.count[h] * bb;
+                K += o.A[h] * o.A[h] * ws[4 * h + 3] + 2.0 * o.A[h] * bs + a.count[h] * bb;
             }
             K *= 0.5 * a.mass;
         }
         const float Kt = (float)(1.5 * a.gas_constant * N * a.target_temperature);
         const float Nf = 3.0f * (float)N;
-        const float R = ok ? (float)randoms[(int64_t)s * a.stride + a.offset + 2 * g] : 0.0f;
-        const float S = ok ? (float)randoms[(int64_t)s * a.stride + a.offset + 2 * g + 1] : Nf - 1.0f;
+        const float R = in.R[g], S = in.S[g];
         const float c = (float)a.c;
         const float q = Kt / (Nf * (float)K);
         const float alpha2 = c + (1.0f - c) * (S + R * R) * q + 2.0f * R * sqrtf(c * (1.0f - c) * q);
         const double al = (double)sqrtf(alpha2);
         if (com) {
-            A[g] *= al;
-            for (int d = 0; d < 3; ++d) B[g][d] = al * (B[g][d] - cnow[d]) + cnow[d];
+            o.A[g] *= al;
+            for (int d = 0; d < 3; ++d) o.B[g][d] = al * (o.B[g][d] - cnow[d]) + cnow[d];
         } else {
-            for (int h = 0; h < ng; ++h) {
-                A[h] *= al;
-                for (int d = 0; d < 3; ++d) B[h][d] *= al;
+            for (int h = 0; h < 2; ++h) {
+                if (h >= ng) break;
+                o.A[h] *= al;
+                for (int d = 0; d < 3; ++d) o.B[h][d] *= al;
             }
         }
-        state[8 + g] += K * ((double)alpha2 - 1.0);
+        o.work[g] = K * ((double)alpha2 - 1.0);
     }
+    return o;
+}
+
+__device__ __forceinline__ void csvr_store(const HpfCsvrArgs& a, const CsvrIn& in,
+                                           const CsvrOut& o, int* counter, double* state) {
+    const int ng = a.n_groups < 1 ? 1 : (a.n_groups > 2 ? 2 : a.n_groups);
     for (int h = 0; h < 2; ++h) {
-        state[4 * h] = A[h];
-        for (int d = 0; d < 3; ++d) state[4 * h + 1 + d] = B[h][d];
+        if (in.act && h < ng) state[8 + h] += o.work[h];
+        state[4 * h] = o.A[h];
+        for (int d = 0; d < 3; ++d) state[4 * h + 1 + d] = o.B[h][d];
     }
-    if (a.advance) *counter = s + 1;
+    if (a.advance) *counter = in.s + 1;
+}
+
+__device__ __forceinline__ void csvr_update(const HpfCsvrArgs& a, const double* ws,
+                                            const double* randoms, int* counter, double* state,
+                                            int* err) {
+    const CsvrIn in = csvr_load(a, randoms, counter, err);
+    csvr_store(a, in, csvr_factors(a, in, ws), counter, state);
 }
 
 // SCR barostat step run by one thread once all sums are final: isotropic

@@ -634,9 +634,10 @@ class RespaMD:
         MD loop's charge paint visits."""
         self.charged = torch.nonzero(self.charges != 0).reshape(-1).to(torch.int32).contiguous()
 
-    def _kick_args(self, thermostat):
+    def _kick_args(self, thermostat, defer=False):
         """HpfKick for the second outer half kick fused into the last readout
-        (with the CSVR sums when the thermostat is on)."""
+        (with the CSVR sums when the thermostat is on; defer: their block
+        partials only, for hpf_csvr_apply)."""
         k = _lib.Kick()
         k.v = self.v.data_ptr()
         if self.charges is not None:
@@ -645,6 +646,7 @@ class RespaMD:
         k.mass = self.mass
         k.dt_outer = self.respa * self.dt
         if thermostat:
+            k.defer = int(defer)
             k.thermo = _lib.ctypes.pointer(self.thermo_args)
             k.group = self.group.data_ptr() if self.group is not None else None
             k.randoms = self.randoms.data_ptr()
@@ -846,11 +848,13 @@ class RespaMD:
             else:
                 self._outer_kick(st)
             return
-        self._field(st, self.field_sums, pos_scale=scale, kick=self._kick_args(thermo),
-                    painted=painted)
+        self._field(st, self.field_sums, pos_scale=scale,
+                    kick=self._kick_args(thermo, defer=True), painted=painted)
         if thermo:
-            _lib.call("hpf_csvr_scale", _lib.ptr(self.v), _lib.ptr(self.group), self.n,
-                      _lib.ptr(self.state), int(self.thermo_args.remove_com), st)
+            _lib.call("hpf_csvr_apply", _lib.ptr(self.v), _lib.ptr(self.group), self.n,
+                      _lib.ctypes.byref(self.thermo_args), _lib.ptr(self.randoms),
+                      _lib.ptr(self.counter), _lib.ptr(self.state), _lib.ptr(self.ws_md),
+                      _lib.ptr(self.err), st)
 
     def capture(self, split=False):
         """Record one outer step in a CUDA graph (after a warm-up step).

@@ -95,12 +95,15 @@ typedef struct {
  * the n_prev slow forces already computed (in order), then for the force
  * this readout produces.  With thermo != NULL the same pass accumulates the
  * per-group velocity sums and the grid's last block forms the CSVR scale
- * factors (as hpf_csvr does, without applying them: call hpf_csvr_scale). */
+ * factors (as hpf_csvr does, without applying them: call hpf_csvr_scale).
+ * With defer != 0 the pass leaves the sums' block partials in ws instead, and
+ * hpf_csvr_apply(v, ..., the same n and ws) forms the factors and applies
+ * them. */
 typedef struct {
     float* v;
     const float* prev[4];
     int n_prev;
-    int pad;
+    int defer;
     double mass, dt_outer;
     const HpfCsvrArgs* thermo;
     const int32_t* group;
@@ -488,6 +491,12 @@ int hpf_csvr(float* v, const int32_t* group, int64_t n, const float* const* kick
 /* kick_forces (n_kick arrays, may be 0): the second outer half kick
  * v += 0.5 kick_dt F/mass (hymd/main.py:1143-1169) applied in the same pass,
  * before the kinetic energy is taken. */
+/* The thermostat after a field evaluation with a deferred kick (HpfKick.defer;
+ * n, ws as there): the factors of hpf_csvr from the velocity sums' partials
+ * in ws, applied to v in the same launch; state, counter as hpf_csvr. */
+int hpf_csvr_apply(float* v, const int32_t* group, int64_t n, const HpfCsvrArgs* args,
+                   const double* randoms, int* counter, double* state, double* ws, int* d_err,
+                   void* stream);
 /* The scaling half of hpf_csvr: v = A_g v + B_g from state
  * (hymd/thermostat.py:210-217); remove_com is carried by the transform in
  * state and is not read. */
