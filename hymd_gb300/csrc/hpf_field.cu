@@ -1423,6 +1423,15 @@ int hpf_field_pic_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
     float* pos_w = painted && pos_scale ? pos : nullptr;
     const double* rscale = painted ? pos_scale : nullptr;
     cudaStream_t st = as_stream(stream);
+    // rRESPA sums still running beside this call: waited for before the
+    // k-space pass, the first kernel here that reads the box; deposits yet to
+    // be made read it too, and with charges both chains follow them
+    cudaEvent_t join = c->pending;
+    c->pending = nullptr;
+    if (join && (!painted || charges)) {
+        HPF_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
+        join = nullptr;
+    }
     int r;
     if (!c->spec_fused) {
         // the library-FFT path shares its plans' work area: one chain after
@@ -1443,7 +1452,7 @@ int hpf_field_pic_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
         if (!painted && (r = do_paint(c, pos, types, nullptr, n, c->T, sc, c->d_grid, st,
                                       pos_scale, false)) != HPF_OK)
             return r;
-        if ((r = spectral_field_force(c, sc.s, sums, st)) != HPF_OK) return r;
+        if ((r = spectral_field_force(c, sc.s, sums, st, join)) != HPF_OK) return r;
         if (n > 0)
             return launch_readout(c, c->d_grid, pos, types, nullptr, n, c->T, force, kick, st,
                                   pos_w, rscale);

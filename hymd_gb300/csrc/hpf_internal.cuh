@@ -98,6 +98,10 @@ struct hpf_ctx {
     double* pic_spec_ws;
     cudaStream_t pic_stream;
     cudaEvent_t pic_fork, pic_join;
+    // the rRESPA sums (and the barostat's box update) still running on their
+    // plan's second stream (hpf_respa_plan_defer): the field step waits for
+    // this event before its k-space pass, then forgets it.  Owned by the plan.
+    cudaEvent_t pending;
 };
 
 // Buffers of one chain of the fused spectral passes: spectra in (pass A ->
@@ -130,7 +134,9 @@ bool spectral_eligible(const hpf_ctx* c);
 int spectral_setup(hpf_ctx* c);
 bool spectral_tile_ok(const hpf_ctx* c, int W);
 int spectral_set_tile(hpf_ctx* c, int W);
-int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st);
+// join (may be NULL): an event that the pass after A waits for.
+int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st,
+                         cudaEvent_t join = nullptr);
 // real_in non-NULL: the input is that real grid (float[M]) instead of the
 // charge accumulator; filter = false drops H(k) from the Poisson map (the GPE
 // solve's psi = scale (q + pol) / k^2).

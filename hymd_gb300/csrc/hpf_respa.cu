@@ -70,6 +70,10 @@ struct hpf_respa_plan {
     // its fork / join events
     cudaStream_t free_stream;
     cudaEvent_t free_fork, free_join;
+    // hpf_respa_plan_defer: the sums run on free_stream after both kernels
+    // (sums_fork) and are joined by the field step (sums_done)
+    int defer;
+    cudaEvent_t sums_fork, sums_done;
 };
 
 namespace {
@@ -803,6 +807,12 @@ int hpf_respa_plan_permute(hpf_respa_plan* p, const int32_t* inv, int64_t n,
     return HPF_OK;
 }
 
+int hpf_respa_plan_defer(hpf_respa_plan* p, int on) {
+    if (!p || on < 0 || on > 1) return HPF_ERR_ARG;
+    p->defer = on;
+    return HPF_OK;
+}
+
 int hpf_respa_plan_counts(const hpf_respa_plan* p, int64_t* n_bonded, int64_t* n_free) {
     if (!p) return HPF_ERR_ARG;
     if (n_bonded) *n_bonded = p->n_bonded;
@@ -821,6 +831,8 @@ int hpf_respa_plan_destroy(hpf_respa_plan* p) {
     if (p->free_stream) cudaStreamDestroy(p->free_stream);
     if (p->free_fork) cudaEventDestroy(p->free_fork);
     if (p->free_join) cudaEventDestroy(p->free_join);
+    if (p->sums_fork) cudaEventDestroy(p->sums_fork);
+    if (p->sums_done) cudaEventDestroy(p->sums_done);
     delete p;
     return HPF_OK;
 }
@@ -1083,6 +1095,8 @@ int hpf_respa_plan_create(hpf_respa_plan** out, int64_t n, int64_t nb, const int
     const int grid = grid_size(p);
     if (cudaMalloc(&p->partials, sizeof(double) * kOut * (size_t)std::max(grid, 1)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&p->free_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&p->sums_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&p->sums_done, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->free_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->free_join, cudaEventDisableTiming) != cudaSuccess) {
         hpf_respa_plan_destroy(p);
@@ -1129,7 +1143,7 @@ int respa_run(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
               int respa_inner, const double* box, float* dipoles, float* transfer, double* out,
               hpf_ctx* baro_ctx, const HpfScrArgs* baro, const double* field_sums,
               const double* randoms, int* counter, double* state, int* d_err, void* stream,
-              const PaintFuse* pf) {
+              const PaintFuse* pf, hpf_ctx* field_ctx) {
     if (!p || !r || !v || !f_bonded || !box || n_slow < 0 || n_slow > kMaxSlow ||
         (n_slow > 0 && !slow_forces) || !(mass > 0) || respa_inner < 1 ||
         (dipoles != nullptr) != (transfer != nullptr))
@@ -1213,6 +1227,18 @@ int respa_run(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
     }
     if (split) HPF_CUDA_TRY(cudaStreamWaitEvent(st, p->free_join, 0));
     if (rc != HPF_OK) return rc;
+    if (out && pf && p->defer) {
+        // the sums (one block, a latency chain) beside the field step's first
+        // pass instead of before it
+        HPF_CUDA_TRY(cudaEventRecord(p->sums_fork, st));
+        HPF_CUDA_TRY(cudaStreamWaitEvent(p->free_stream, p->sums_fork, 0));
+        const cudaError_t e =
+            launch_pdl(k_respa_finish, 1, kFinishThreads, 0, p->free_stream,
+                       static_cast<const double*>(p->partials), G, out, bf, d_err);
+        HPF_CUDA_TRY(cudaEventRecord(p->sums_done, p->free_stream));
+        field_ctx->pending = p->sums_done;
+        return e == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
+    }
     if (out && launch_pdl(k_respa_finish, 1, kFinishThreads, 0, st,
                           static_cast<const double*>(p->partials), G, out, bf, d_err) !=
                    cudaSuccess)
@@ -1232,7 +1258,7 @@ int hpf_respa_step(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
                    int* d_err, void* stream) {
     return respa_run(p, r, v, f_bonded, slow_forces, n_slow, mass, dt, respa_inner, box, dipoles,
                      transfer, out, baro_ctx, baro, field_sums, randoms, counter, state, d_err,
-                     stream, nullptr);
+                     stream, nullptr, nullptr);
 }
 
 int hpf_respa_step_paint(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
@@ -1256,7 +1282,7 @@ int hpf_respa_step_paint(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
     pf.err = d_err ? d_err : field_ctx->d_err;
     return respa_run(p, r, v, f_bonded, slow_forces, n_slow, mass, dt, respa_inner, box, dipoles,
                      transfer, out, baro ? field_ctx : nullptr, baro, field_sums, randoms, counter,
-                     state, d_err, stream, &pf);
+                     state, d_err, stream, &pf, field_ctx);
 }
 
 int hpf_respa_forces(hpf_respa_plan* p, const float* r, float* f_bonded, const double* box,

@@ -116,12 +116,15 @@ __device__ __forceinline__ int plane_row(int r) {
 // the half spectrum X[0..h] fused into the first step of the y transform;
 // the y transform's second step writes the spectrum plane.
 // blockIdx.y: the grid (type) of acc and spec; sc.s[that grid] scales it.
+// The accumulators become painted weights per cell here; the division by the
+// cell volume is pass B's, so that this pass does not need the box and can
+// run while a barostat still updates it.
 // FIX = false: the input is a real grid (fin, float[grids][M]) scaled by
 // sc.s[grid] alone, read and left as it is (the accumulators are not used).
 template <int NY, int HZ, bool FIX = true>
 __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_fwd(unsigned long long* __restrict__ acc, float2* __restrict__ spec, SpecGeom g,
-               SpecScale sc, const BoxState* __restrict__ bs, const float2* __restrict__ tw,
+               SpecScale sc, const float2* __restrict__ tw,
                const float* __restrict__ fin = nullptr) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto zs = [](int e) { return PN > 1 ? e + e / PN : e; };
     auto row0 = [](int r) { return plane_row<NY, HZ>(r); };
-    const float s = FIX ? sc.s[t] * bs->inv_dV * kFixInv : sc.s[t];
+    const float s = FIX ? sc.s[t] * kFixInv : sc.s[t];
     ulonglong2* a =
         FIX ? reinterpret_cast<ulonglong2*>(acc + (int64_t)t * g.M + (int64_t)x * Ny * (2 * H))
             : nullptr;
@@ -249,7 +252,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     tile_columns(col, g, j0, bs);
     using fx = Idx<N>;
     const float kf0 = bs->kf[0];
-    const float invM = (float)bs->inv_M;
+    // 1 / M of the unnormalised transform, and the weights' 1 / dV
+    const float invM = (float)bs->inv_M * bs->inv_dV;
     const float s2h = fun->sigma2_half;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     const int cin = T * W, cout = 2 * T * W;
@@ -384,7 +388,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_kspace_pic(const float2* __restrict__ rho, float2* __restrict__ out_spec, SpecGeom g,
                       const BoxState* __restrict__ bs, const Functional* __restrict__ fun,
                       float four_pi_fac, const float2* __restrict__ tw,
-                      double* sums, double* partials, unsigned int* ticket, int filter) {
+                      double* sums, double* partials, unsigned int* ticket, int filter,
+                      int by_volume) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
     __shared__ ColInfo col[16];
@@ -396,7 +401,9 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     tile_columns(col, g, j0, bs);
     using fx = Idx<N>;
     const float kf0 = bs->kf[0];
-    const float invM = (float)bs->inv_M;
+    // by_volume: the input spectrum is that of weights per cell (a real grid
+    // holds densities)
+    const float invM = by_volume ? (float)bs->inv_M * bs->inv_dV : (float)bs->inv_M;
     const float s2h = fun->sigma2_half;
     float acc[1] = {0.0f};
     const int cout = 2 * W;
@@ -751,18 +758,20 @@ size_t spectral_ws_words(const hpf_ctx* c) { return 4 * (size_t)c->spec_max_tile
 
 // accumulators (T grids, painted) -> force mesh c->d_grid [3T][M]; sums as
 // k_kspace_force's (out[0..3]) when non-null.
-int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st) {
+int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st,
+                         cudaEvent_t join) {
     const SpecGeom g = spec_geom(c, c->spec_W);
     SpecScale sc;
     for (int t = 0; t < c->T; ++t) sc.s[t] = type_scale[t];
     const int ps = (int)plane_smem(c), ts = (int)tile_smem(c, g.W);
     if (with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto) {
             return launch_pdl(kf, dim3(c->n0, c->T), kSpecThreads, ps, st, c->d_acc,
-                              c->d_spec_phi, g, sc, c->d_box, c->d_tw, nullptr) == cudaSuccess
+                              c->d_spec_phi, g, sc, c->d_tw, nullptr) == cudaSuccess
                        ? HPF_OK
                        : HPF_ERR_CUDA;
         }) != HPF_OK)
         return HPF_ERR_CUDA;
+    if (join) HPF_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
     double* part = c->d_spec_ws;
     unsigned int* tick = reinterpret_cast<unsigned int*>(c->d_spec_ws + 4 * (size_t)c->spec_max_tiles);
     int r = with_kspace(c->n0, [&](auto kd, auto) {
@@ -795,10 +804,10 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
     if (with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto kr) {
             const cudaError_t e =
                 real_in ? launch_pdl(kr, dim3(c->n0, 1), kSpecThreads, ps, st, nullptr,
-                                     b.spec_phi, g, sc, c->d_box, c->d_tw, real_in)
+                                     b.spec_phi, g, sc, c->d_tw, real_in)
                         : launch_pdl(kf, dim3(c->n0, 1), kSpecThreads, ps, st,
                                      c->d_acc + (int64_t)c->T * c->M, b.spec_phi, g, sc,
-                                     c->d_box, c->d_tw, nullptr);
+                                     c->d_tw, nullptr);
             return e == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
         }) != HPF_OK)
         return HPF_ERR_CUDA;
@@ -807,7 +816,7 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
     int r = with_kspace(c->n0, [&](auto, auto kp) {
         return launch_pdl(kp, c->spec_tiles_pic, kSpecThreads, ts, st, b.spec_phi, b.spec, g,
                           c->d_box, c->d_fun, four_pi_fac, c->d_tw, sums, part, tick,
-                          filter ? 1 : 0) == cudaSuccess
+                          filter ? 1 : 0, real_in ? 0 : 1) == cudaSuccess
                    ? HPF_OK
                    : HPF_ERR_CUDA;
     });
