@@ -429,7 +429,7 @@ __global__ void k_paint_finalize_f64(unsigned long long* __restrict__ acc,
 template <int TT>
 __global__ void k_energy_f64(const double2* __restrict__ spec, int T_rt, int has_q, int64_t Mc,
                              KGeom g, double invM, const BoxState* __restrict__ bs,
-                             const Functional* __restrict__ fun, TypeScale qt, double four_pi_fac,
+                             const Functional* __restrict__ fun, TypeScaleD qt, double four_pi_fac,
                              double* out, double* partials, unsigned int* ticket) {
     constexpr int TM = TT > 0 ? TT : HPF_MAX_TYPES;
     const int T = TT > 0 ? TT : T_rt;
@@ -490,7 +490,7 @@ __global__ void k_energy_f64(const double2* __restrict__ spec, int T_rt, int has
             const double2 psi = make_double2(rho.x * s, rho.y * s);
             acc[4] += wk * (rho.x * psi.x + rho.y * psi.y);
             double cr = 0.0;
-            for (int t = 0; t < T; ++t) cr += (double)qt.s[t] * (psi.x * ph[t].x + psi.y * ph[t].y);
+            for (int t = 0; t < T; ++t) cr += qt.s[t] * (psi.x * ph[t].x + psi.y * ph[t].y);
             acc[5] += wk * cr;
             for (int d = 0; d < 3; ++d) acc[6 + d] += wk * kk[d] * cr;
         }
@@ -697,13 +697,21 @@ int grid_for(int64_t work, int threads) {
     return (int)(b < cap ? b : cap);
 }
 
+int ensure_spec64(hpf_ctx* c) {
+    if (c->d_spec64) return HPF_OK;
+    HPF_CUDA_TRY(cudaMalloc(&c->d_spec64, sizeof(double2) * (size_t)(c->T + 1) * c->Mc));
+    return HPF_OK;
+}
+
 // The FP64 buffers and the D2Z plan (batch T+1: densities + charges) are
 // only needed for energies and gradients: created on first use.
 int ensure_d2z(hpf_ctx* c) {
     if (c->has_d2z) return HPF_OK;
     const int T = c->T;
-    HPF_CUDA_TRY(cudaMalloc(&c->d_grid64, sizeof(double) * (size_t)(T + 1) * c->M));
-    HPF_CUDA_TRY(cudaMalloc(&c->d_spec64, sizeof(double2) * (size_t)(T + 1) * c->Mc));
+    if (!c->d_grid64)
+        HPF_CUDA_TRY(cudaMalloc(&c->d_grid64, sizeof(double) * (size_t)(T + 1) * c->M));
+    int r = ensure_spec64(c);
+    if (r != HPF_OK) return r;
     long long nn[3] = {c->n0, c->n1, c->n2};
     size_t ws = 0;
     if (cufftCreate(&c->plan_d2z) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
@@ -713,6 +721,22 @@ int ensure_d2z(hpf_ctx* c) {
         return HPF_ERR_CUFFT;
     }
     c->has_d2z = true;
+    return HPF_OK;
+}
+
+// Deposits of the densities, and of the charges into slot T when given.
+int paint_f64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n, const float* charges,
+              cudaStream_t st) {
+    if (n <= 0) return HPF_OK;
+    k_paint<<<grid_for(n, kThreads), kThreads, 0, st>>>(pos, types, nullptr, n, c->T, c->d_box,
+                                                       c->d_acc, c->M, c->d_err, nullptr);
+    HPF_LAUNCH_CHECK();
+    if (charges) {
+        k_paint<<<grid_for(n, kThreads), kThreads, 0, st>>>(
+            pos, nullptr, charges, n, 1, c->d_box, c->d_acc + (int64_t)c->T * c->M, c->M, c->d_err,
+            nullptr);
+        HPF_LAUNCH_CHECK();
+    }
     return HPF_OK;
 }
 
@@ -726,17 +750,7 @@ int density_spectra_f64(hpf_ctx* c, const float* pos, const int32_t* types, int6
     TypeScaleD sc;
     for (int t = 0; t < T; ++t) sc.s[t] = type_mass[t];
     sc.s[T] = 1.0;
-    if (n > 0) {
-        k_paint<<<grid_for(n, kThreads), kThreads, 0, st>>>(pos, types, nullptr, n, T, c->d_box,
-                                                           c->d_acc, c->M, c->d_err, nullptr);
-        HPF_LAUNCH_CHECK();
-        if (charges) {
-            k_paint<<<grid_for(n, kThreads), kThreads, 0, st>>>(
-                pos, nullptr, charges, n, 1, c->d_box, c->d_acc + (int64_t)T * c->M, c->M,
-                c->d_err, nullptr);
-            HPF_LAUNCH_CHECK();
-        }
-    }
+    if ((r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK) return r;
     k_paint_finalize_f64<<<grid_for((int64_t)(T + 1) * c->M, kThreads), kThreads, 0, st>>>(
         c->d_acc, c->d_grid64, c->M, T + 1, sc, c->d_box);
     HPF_LAUNCH_CHECK();
@@ -957,6 +971,7 @@ int hpf_ctx_destroy(hpf_ctx* c) {
     if (c->gpe_graph) cudaGraphDestroy(c->gpe_graph);
     if (c->gpe_cap) cudaStreamDestroy(c->gpe_cap);
     cudaFree(c->d_tw);
+    cudaFree(c->df_tw);
     cudaFree(c->d_spec_ws);
     cudaFree(c->pic_spec_phi);
     cudaFree(c->pic_spec);
@@ -1203,10 +1218,19 @@ int hpf_energy_fp64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t 
     if (!c || !type_mass || !out || n < 0 || (n > 0 && (!pos || !types))) return HPF_ERR_ARG;
     cudaStream_t st = as_stream(stream);
     const int T = c->T;
+    if (energy_df_ok(c)) {
+        int r;
+        if ((r = ensure_spec64(c)) != HPF_OK || (r = energy_df_setup(c)) != HPF_OK ||
+            (r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK)
+            return r;
+        return energy_df(c, charges ? T + 1 : T, type_mass, type_charges,
+                         4.0 * 3.14159265358979323846 * elec_factor,
+                         reinterpret_cast<float4*>(c->d_spec64), out, st);
+    }
     int r0 = density_spectra_f64(c, pos, types, n, type_mass, charges, st);
     if (r0 != HPF_OK) return r0;
-    TypeScale qt;
-    for (int t = 0; t < T; ++t) qt.s[t] = type_charges ? (float)type_charges[t] : 0.0f;
+    TypeScaleD qt;
+    for (int t = 0; t < T; ++t) qt.s[t] = type_charges ? type_charges[t] : 0.0;
     KGeom g = kgeom(c);
     int grid = reduce_grid(c->Mc, kThreads);
     if (grid > 896) grid = 896;  // 9 partials per block must fit the workspace

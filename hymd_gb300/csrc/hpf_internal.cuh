@@ -83,6 +83,7 @@ struct hpf_ctx {
     // fused spectral passes: twiddle tables exp(-2 pi i m / 512) and
     // exp(-2 pi i m / 768), k-space tile width, partial sums + ticket
     float2* d_tw;
+    float4* df_tw;  // double-float twiddles and scratch (energy_df_setup)
     double* d_spec_ws;
     int spec_W, spec_tiles, spec_max_tiles;
     int spec_W_pic, spec_tiles_pic;  // the charge k-space pass's own tile width
@@ -142,6 +143,12 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
 // solve's psi = scale (q + pol) / k^2).
 int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi, double* sums,
                  cudaStream_t st, const float* real_in = nullptr, bool filter = true);
+// FP64 energy sums in double-float arithmetic (hpf_energy.cu): whether they
+// apply, setup on first use, painted accumulators (G grids) -> out[32].
+bool energy_df_ok(const hpf_ctx* c);
+int energy_df_setup(hpf_ctx* c);
+int energy_df(hpf_ctx* c, int G, const double* type_mass, const double* type_charges,
+              double four_pi_fac, float4* spec, double* out, cudaStream_t st);
 // words of a pass-B partial-sum buffer (partials of the narrowest tile + ticket)
 size_t spectral_ws_words(const hpf_ctx* c);
 
