@@ -119,6 +119,8 @@ _SIGNATURES.update({
     "hpf_field_adjoint": [P, P, P, I64, ctypes.POINTER(D), P, P, P],
     "hpf_scr_scale_positions": [P, I64, P, I, P],
     "hpf_respa_forces": [P, P, P, P, P, P, P],
+    "hpf_respa_vjp_ok": [P, ctypes.POINTER(I)],
+    "hpf_respa_vjp": [P, P, P, P, ctypes.POINTER(P), I, D, D, I, P, P, P, P, P, P, P],
     "hpf_pic_force_vjp": [P, P, P, I64, D, P, P, P],
     "hpf_field_force_vjp": [P, P, P, I64, ctypes.POINTER(D), P, P, P, P],
     "hpf_dihedral_hvp": [P, P, P, I64, P, P, P, P, P, P, P, P, I64, P, P],

@@ -27,6 +27,7 @@
 #include <numeric>
 #include <vector>
 
+#include "hpf_dual.cuh"
 #include "hpf_internal.cuh"
 #include "hpf_terms.cuh"
 
@@ -630,6 +631,258 @@ k_respa_cta(hpf_respa_plan p, float* __restrict__ r, float* __restrict__ v,
     if (out) block_partials_f<kOut, kThreads>(acc, p.partials, G);
 }
 
+// Reverse mode of the whole inner loop of one group.  The forward loop is run
+// again from its inputs, each drift's positions going to `traj` (global,
+// [inner step][group bead]; a bead is written and read by the same lane), and
+// then walked backwards: with (X, V) the cotangents of (x_s, v_s) and h =
+// dt / 2m,
+//   L = cotangent of f_s + h V,  X += J(x_s) L,  V += dt X,
+// where J, the (symmetric) Jacobian of the bonded forces, is applied term by
+// term by the forward derivative along L; the terms' contributions pass
+// through the force slots, so the sums have a fixed order.  The cotangent of
+// f_s is h V of the step after it (f_s also opens that step); the gradient
+// with respect to the loop's own input force is h V.
+// One launch where the step-by-step form needs several kernels and a dozen
+// tensor operations for each of the respa_inner steps: that form is bound by
+// its launches (differentiated trajectory of a 40k-bead membrane: 2 steps of
+// 10 inner steps, forward and backward, 15.7 ms).
+struct VjpArgs {
+    float *gx, *gv, *gf;  // cotangents of the outputs; gradients on return
+    float* gslow;         // gradient of the sum of the slow forces, or NULL
+    float4* traj;
+    int64_t n_bonded;
+};
+
+template <bool DIH, typename Sync>
+__device__ __forceinline__ void vjp_group(const hpf_respa_plan& p, int grp, int lane, int width,
+                                          char* smem_base, const float* __restrict__ r,
+                                          const float* __restrict__ v,
+                                          const float* __restrict__ fb, const SlowForces& slow,
+                                          float mass, float h_out, float hdt, float dt, int respa,
+                                          const Box& bx, const VjpArgs& a, Sync sync) {
+    const GroupSmem s = carve(smem_base, p);
+    float4* adj_v = reinterpret_cast<float4*>(smem_base + p.smem_group);
+    const int s0 = p.grp_bead[grp], nb = p.grp_bead[grp + 1] - s0;
+    const int b0 = p.grp_bond[grp], nbd = p.grp_bond[grp + 1] - b0;
+    const int a0 = p.grp_ang[grp], na = p.grp_ang[grp + 1] - a0;
+    const int d0 = DIH ? p.grp_dih[grp] : 0, nd = DIH ? p.grp_dih[grp + 1] - d0 : 0;
+    const int i0 = p.bead_inc[s0];
+    const float inv_m = 1.0f / mass;
+    for (int i = lane; i < nb; i += width) {
+        const int64_t g = 3 * (int64_t)p.bead_ids[s0 + i];
+        float xv[3], xr[3], xf[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            float x = v[g + d];
+#pragma unroll
+            for (int q = 0; q < kMaxSlow; ++q)
+                if (q < slow.n) x = x + h_out * div_m(slow.f[q][g + d], mass, inv_m);
+            xv[d] = x;
+            xr[d] = r[g + d];
+            xf[d] = fb[g + d];
+        }
+        s.vs[i] = make_float4(xv[0], xv[1], xv[2], 0.0f);
+        s.rs[i] = make_float4(xr[0], xr[1], xr[2], 0.0f);
+        s.fs[i] = make_float4(xf[0], xf[1], xf[2], 0.0f);
+    }
+    for (int t = lane; t < nbd; t += width) {
+        s.bond_ij[t] = p.bond_ij[b0 + t];
+        s.bond_p[t] = p.bond_p[b0 + t];
+    }
+    for (int t = lane; t < na; t += width) {
+        s.ang_ijk[t] = p.ang_ijk[a0 + t];
+        s.ang_p[t] = p.ang_p[a0 + t];
+    }
+    for (int i = lane; i <= nb; i += width) s.inc_start[i] = p.bead_inc[s0 + i] - i0;
+    const int ninc = p.bead_inc[s0 + nb] - i0;
+    for (int t = lane; t < ninc; t += width) s.inc[t] = p.inc_list[i0 + t];
+    sync();
+    auto gather = [&](int i) {
+        float4 F = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int q = s.inc_start[i]; q < s.inc_start[i + 1]; ++q) {
+            const int en = s.inc[q];
+            const float4 sl = s.slot[en >> 1];
+            const float sg = (en & 1) ? -1.0f : 1.0f;
+            F.x = fmaf(sg, sl.x, F.x);
+            F.y = fmaf(sg, sl.y, F.y);
+            F.z = fmaf(sg, sl.z, F.z);
+        }
+        return F;
+    };
+    // forward: positions after each drift (the forces of the last one are not
+    // needed)
+    for (int it = 0; it < respa; ++it) {
+        for (int i = lane; i < nb; i += width) {
+            const float4 F = it == 0 ? s.fs[i] : gather(i);
+            const float4 vv = s.vs[i], rv = s.rs[i];
+            float xr[3] = {rv.x, rv.y, rv.z}, xv[3] = {vv.x, vv.y, vv.z};
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float acc = div_m(comp(F, d), mass, inv_m);
+                float x = xv[d];
+                if (it > 0) x = x + hdt * acc;
+                x = x + hdt * acc;
+                xr[d] = wrapf(xr[d] + dt * x, bx.L[d]);
+                xv[d] = x;
+            }
+            s.vs[i] = make_float4(xv[0], xv[1], xv[2], 0.0f);
+            s.rs[i] = make_float4(xr[0], xr[1], xr[2], 0.0f);
+            a.traj[(int64_t)it * a.n_bonded + s0 + i] = s.rs[i];
+        }
+        sync();
+        if (it == respa - 1) break;
+        for (int t = lane; t < nbd; t += width) {
+            const int ij = s.bond_ij[t];
+            float e;
+            V3 vir;
+            put3(s.slot, t, bond_term(get3(s.rs, ij & 0xffff), get3(s.rs, ij >> 16),
+                                      s.bond_p[t].x, s.bond_p[t].y, bx, e, vir));
+        }
+        for (int t = lane; t < na; t += width) {
+            const int2 q = s.ang_ijk[t];
+            V3 ga, gc, vir;
+            float e;
+            if (!angle_term(get3(s.rs, q.x & 0xffff), get3(s.rs, q.x >> 16), get3(s.rs, q.y),
+                            s.ang_p[t].x, s.ang_p[t].y, bx, ga, gc, e, vir))
+                ga = gc = v3(0.f, 0.f, 0.f);
+            put3(s.slot, nbd + t, ga);
+            put3(s.slot, nbd + na + t, gc);
+        }
+        if (DIH) {
+            for (int t = lane; t < nd; t += width) {
+                const short4 q = p.dih_ijkl[d0 + t];
+                const int2 tl = p.dih_tl[d0 + t];
+                const int64_t c30 = 30 * (int64_t)(d0 + t);
+                V3 F[4];
+                float e;
+                dihedral_term(get3(s.rs, q.x), get3(s.rs, q.y), get3(s.rs, q.z), get3(s.rs, q.w),
+                              p.dih_coeff + c30, p.dih_trig + c30, tl.x, tl.y, 0, bx, F, e, nullptr,
+                              nullptr);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) put3(s.slot, nbd + 2 * na + t + j * nd, F[j]);
+            }
+        }
+        sync();
+    }
+    // backward; X in fs, V in adj_v, L in vs, x_s in rs
+    const float h = hdt * inv_m;
+    for (int i = lane; i < nb; i += width) {
+        const int64_t g = 3 * (int64_t)p.bead_ids[s0 + i];
+        s.fs[i] = make_float4(a.gx[g], a.gx[g + 1], a.gx[g + 2], 0.0f);
+        const float4 V = make_float4(a.gv[g], a.gv[g + 1], a.gv[g + 2], 0.0f);
+        adj_v[i] = V;
+        s.vs[i] = make_float4(fmaf(h, V.x, a.gf[g]), fmaf(h, V.y, a.gf[g + 1]),
+                              fmaf(h, V.z, a.gf[g + 2]), 0.0f);
+    }
+    sync();
+    for (int it = respa - 1; it >= 0; --it) {
+        for (int t = lane; t < nbd; t += width) {
+            const int ij = s.bond_ij[t], bi = ij & 0xffff, bj = ij >> 16;
+            put3(s.slot, t, bond_force_tangent(get3(s.rs, bi), get3(s.rs, bj), get3(s.vs, bi),
+                                               get3(s.vs, bj), s.bond_p[t].x, s.bond_p[t].y, bx));
+        }
+        for (int t = lane; t < na; t += width) {
+            const int2 q = s.ang_ijk[t];
+            const int ai = q.x & 0xffff, aj = q.x >> 16, ak = q.y;
+            V3 dga, dgc;
+            if (!angle_grad_tangent(get3(s.rs, ai), get3(s.rs, aj), get3(s.rs, ak),
+                                    get3(s.vs, ai), get3(s.vs, aj), get3(s.vs, ak), s.ang_p[t].x,
+                                    s.ang_p[t].y, bx, dga, dgc))
+                dga = dgc = v3(0.f, 0.f, 0.f);
+            put3(s.slot, nbd + t, dga);
+            put3(s.slot, nbd + na + t, dgc);
+        }
+        if (DIH) {
+            for (int t = lane; t < nd; t += width) {
+                const short4 q = p.dih_ijkl[d0 + t];
+                const int2 tl = p.dih_tl[d0 + t];
+                const int64_t c30 = 30 * (int64_t)(d0 + t);
+                V3 dF[4];
+                dihedral_force_tangent(get3(s.rs, q.x), get3(s.rs, q.y), get3(s.rs, q.z),
+                                       get3(s.rs, q.w), get3(s.vs, q.x), get3(s.vs, q.y),
+                                       get3(s.vs, q.z), get3(s.vs, q.w), p.dih_coeff + c30,
+                                       p.dih_trig + c30, tl.x, tl.y, bx, dF);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) put3(s.slot, nbd + 2 * na + t + j * nd, dF[j]);
+            }
+        }
+        sync();
+        for (int i = lane; i < nb; i += width) {
+            const float4 J = gather(i);
+            float4 X = s.fs[i], V = adj_v[i];
+            X.x += J.x;
+            X.y += J.y;
+            X.z += J.z;
+            V.x = fmaf(dt, X.x, V.x);
+            V.y = fmaf(dt, X.y, V.y);
+            V.z = fmaf(dt, X.z, V.z);
+            s.fs[i] = X;
+            adj_v[i] = V;
+            // the force before this drift: closes the step before (h V) and
+            // opens this one (h V)
+            const float w = it > 0 ? 2.0f * h : h;
+            s.vs[i] = make_float4(w * V.x, w * V.y, w * V.z, 0.0f);
+            if (it > 0) s.rs[i] = a.traj[(int64_t)(it - 1) * a.n_bonded + s0 + i];
+        }
+        sync();
+    }
+    const float hs = h_out * inv_m;
+    for (int i = lane; i < nb; i += width) {
+        const int64_t g = 3 * (int64_t)p.bead_ids[s0 + i];
+        const float4 X = s.fs[i], V = adj_v[i], F = s.vs[i];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            a.gx[g + d] = comp(X, d);
+            a.gv[g + d] = comp(V, d);
+            a.gf[g + d] = comp(F, d);
+            if (a.gslow) a.gslow[g + d] = hs * comp(V, d);
+        }
+    }
+}
+
+// Free beads: x' = x + respa dt v, v' = v + slow kicks; their bonded force is
+// passed through.
+__device__ __forceinline__ void vjp_free(const hpf_respa_plan& p, int fblock, int blocks,
+                                         float mass, float h_out, float dt, int respa,
+                                         const VjpArgs& a) {
+    const float hs = h_out / mass;
+    for (int j = fblock * kThreads + threadIdx.x; j < p.n_free; j += blocks * kThreads) {
+        const int64_t g = 3 * (int64_t)p.free_ids[j];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float X = a.gx[g + d];
+            float V = a.gv[g + d];
+            for (int it = 0; it < respa; ++it) V = fmaf(dt, X, V);
+            a.gv[g + d] = V;
+            if (a.gslow) a.gslow[g + d] = hs * V;
+        }
+    }
+}
+
+template <bool DIH, bool CTA>
+__global__ void __launch_bounds__(kThreads)
+k_respa_vjp(hpf_respa_plan p, const float* __restrict__ r, const float* __restrict__ v,
+            const float* __restrict__ fb, SlowForces slow, float mass, float h_out, float hdt,
+            float dt, int respa, const double* __restrict__ box, VjpArgs a, int n_grp_blocks,
+            size_t smem_group) {
+    extern __shared__ __align__(16) char smem[];
+    const Box bx = load_box(box);
+    if ((int)blockIdx.x < n_grp_blocks) {
+        if (CTA) {
+            vjp_group<DIH>(p, blockIdx.x, threadIdx.x, kThreads, smem, r, v, fb, slow, mass, h_out,
+                           hdt, dt, respa, bx, a, CtaSync());
+        } else {
+            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const int grp = blockIdx.x * kWarps + warp;
+            if (grp < p.n_groups)
+                vjp_group<DIH>(p, grp, lane, 32, smem + (size_t)warp * smem_group, r, v, fb, slow,
+                               mass, h_out, hdt, dt, respa, bx, a, WarpSync());
+        }
+    } else {
+        vjp_free(p, blockIdx.x - n_grp_blocks, gridDim.x - n_grp_blocks, mass, h_out, dt, respa, a);
+    }
+}
+
 // The free beads of a split launch, beside the group kernel (on a second
 // stream): the free-bead blocks of k_respa_warp / k_respa_cta with the same
 // beads per block, without the groups' dynamic shared memory, so that they
@@ -773,6 +1026,13 @@ int upload(T** dst, const std::vector<T>& src) {
         cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return HPF_ERR_CUDA;
     return HPF_OK;
+}
+
+// Dynamic shared memory of a block of k_respa_vjp: the group layout and the
+// velocity cotangents.
+size_t vjp_smem(const hpf_respa_plan* p) {
+    if (p->n_groups == 0) return 0;
+    return (p->smem_group + sizeof(float4) * p->mx_beads) * (p->warp_mode ? kWarps : 1);
 }
 
 int grid_size(const hpf_respa_plan* p) {
@@ -1283,6 +1543,48 @@ int hpf_respa_step_paint(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
     return respa_run(p, r, v, f_bonded, slow_forces, n_slow, mass, dt, respa_inner, box, dipoles,
                      transfer, out, baro ? field_ctx : nullptr, baro, field_sums, randoms, counter,
                      state, d_err, stream, &pf, field_ctx);
+}
+
+int hpf_respa_vjp_ok(const hpf_respa_plan* p, int* ok) {
+    if (!p || !ok) return HPF_ERR_ARG;
+    *ok = vjp_smem(p) <= 227 * 1024;
+    return HPF_OK;
+}
+
+int hpf_respa_vjp(hpf_respa_plan* p, const float* r, const float* v, const float* f_bonded,
+                  const float* const* slow_forces, int n_slow, double mass, double dt,
+                  int respa_inner, const double* box, float* gx, float* gv, float* gf,
+                  float* gslow, void* traj, void* stream) {
+    if (!p || !r || !v || !f_bonded || !box || !gx || !gv || !gf || n_slow < 0 ||
+        n_slow > kMaxSlow || (n_slow > 0 && !slow_forces) || !(mass > 0) || respa_inner < 1 ||
+        (p->n_bonded > 0 && (!traj || (reinterpret_cast<uintptr_t>(traj) & 15))))
+        return HPF_ERR_ARG;
+    SlowForces sf;
+    sf.n = n_slow;
+    for (int q = 0; q < n_slow; ++q) {
+        if (!slow_forces[q]) return HPF_ERR_ARG;
+        sf.f[q] = slow_forces[q];
+    }
+    const int gb = p->warp_mode ? (p->n_groups + kWarps - 1) / kWarps : p->n_groups;
+    const int fbl = std::min((p->n_free + kThreads - 1) / kThreads, 8 * 152);
+    if (gb + fbl == 0) return HPF_OK;
+    const size_t per = p->smem_group + sizeof(float4) * p->mx_beads;
+    const size_t smem = vjp_smem(p);
+    if (smem > 227 * 1024) return HPF_ERR_NOT_IMPLEMENTED;
+    const VjpArgs a{gx, gv, gf, gslow, reinterpret_cast<float4*>(traj), p->n_bonded};
+    const float h_out = (float)(0.5 * respa_inner * dt), hdt = (float)(0.5 * dt);
+    cudaStream_t st = as_stream(stream);
+    auto run = [&](auto k) {
+        if (smem > 48 * 1024 &&
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
+                cudaSuccess)
+            return HPF_ERR_CUDA;
+        k<<<gb + fbl, kThreads, smem, st>>>(*p, r, v, f_bonded, sf, (float)mass, h_out, hdt,
+                                            (float)dt, respa_inner, box, a, gb, per);
+        return cudaGetLastError() == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
+    };
+    if (p->warp_mode) return p->has_dih ? run(k_respa_vjp<true, false>) : run(k_respa_vjp<false, false>);
+    return p->has_dih ? run(k_respa_vjp<true, true>) : run(k_respa_vjp<false, true>);
 }
 
 int hpf_respa_forces(hpf_respa_plan* p, const float* r, float* f_bonded, const double* box,

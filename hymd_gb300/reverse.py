@@ -23,6 +23,9 @@ kernels in libhpf_gb300.so:
     bending force where the reference clamps sin(gamma) at 0.1
     (dipole_reconstruction.f90): there its force is not the gradient of its
     energy, and the product is that of the energy's Hessian;
+  * the inner loop as a whole (first outer half kick, respa_inner drifts,
+    wraps and half kicks with the bonded forces): forward hpf_respa_step,
+    backward hpf_respa_vjp, one launch each;
   * the CSVR thermostat (hymd/thermostat.py:111-219) at the end of the outer
     step, when the RespaMD is coupled, with the random numbers of its table
     (row = step index), as torch operations.
@@ -71,6 +74,14 @@ class ForceModel:
         self.box = md.box
         self.box_f = md.box.float()
         self._key = None
+        # the inner loop as one launch each way (hpf_respa_vjp); a molecule
+        # too large for its shared memory keeps the step-by-step form
+        ok = _lib.I(0)
+        _lib.call("hpf_respa_vjp_ok", md.plan, _lib.ctypes.byref(ok))
+        self.fused_inner = bool(ok.value)
+        nb, nf = _lib.I64(), _lib.I64()
+        _lib.call("hpf_respa_plan_counts", md.plan, _lib.ctypes.byref(nb), _lib.ctypes.byref(nf))
+        self.n_bonded = nb.value
         # PIC_Spectral electrostatics of a charged RespaMD
         self.charges = md.charges
         self.elec_factor = float(md.elec_factor) if md.charges is not None else 0.0
@@ -186,6 +197,40 @@ class _PicForce(torch.autograd.Function):
         return g, None
 
 
+class _InnerLoop(torch.autograd.Function):
+    """The first outer half kick and the respa_inner inner steps of one outer
+    step (hymd/main.py:802-887): hpf_respa_step forward, hpf_respa_vjp
+    backward."""
+
+    @staticmethod
+    def forward(ctx, x, v, f_slow, f_bond, model):
+        md = model.md
+        x, v, f_slow, f_bond = (t.contiguous() for t in (x, v, f_slow, f_bond))
+        r, w, fb = x.clone(), v.clone(), f_bond.clone()
+        arr = (_lib.P * 1)(_lib.ptr(f_slow))
+        _lib.call("hpf_respa_step", md.plan, _lib.ptr(r), _lib.ptr(w), _lib.ptr(fb), arr, 1,
+                  md.mass, md.dt, md.respa, _lib.ptr(model.box), None, None, None, None, None,
+                  None, None, None, None, _lib.ptr(md.err), _lib.stream_ptr())
+        ctx.model = model
+        ctx.save_for_backward(x, v, f_slow, f_bond)
+        return r, w, fb
+
+    @staticmethod
+    def backward(ctx, gx, gv, gf):
+        x, v, f_slow, f_bond = ctx.saved_tensors
+        model = ctx.model
+        md = model.md
+        # overwritten with the inputs' gradients
+        gx, gv, gf = (t.contiguous().clone() for t in (gx, gv, gf))
+        gs = torch.empty_like(gx)
+        traj = torch.empty((md.respa, model.n_bonded, 4), dtype=torch.float32, device=x.device)
+        arr = (_lib.P * 1)(_lib.ptr(f_slow))
+        _lib.call("hpf_respa_vjp", md.plan, _lib.ptr(x), _lib.ptr(v), _lib.ptr(f_bond), arr, 1,
+                  md.mass, md.dt, md.respa, _lib.ptr(model.box), _lib.ptr(gx), _lib.ptr(gv),
+                  _lib.ptr(gf), _lib.ptr(gs), _lib.ptr(traj), _lib.stream_ptr())
+        return gx, gv, gs, gf, None
+
+
 def field_force(x, chi, model):
     """The slow force of the outer kicks: the field force, plus the
     PIC_Spectral electrostatic force of a charged system."""
@@ -236,19 +281,23 @@ def csvr(v, model, step):
 
 
 def respa_step(x, v, f_field, f_bond, chi, model, step=None):
-    """One outer rRESPA step (hymd/main.py:802-887, 1143-1169) in torch
-    operations: outer half kick, respa_inner x (half kick, drift, wrap,
-    bonded forces, half kick), field forces, outer half kick, and the CSVR
-    thermostat of outer step `step` when the RespaMD is coupled."""
+    """One outer rRESPA step (hymd/main.py:802-887, 1143-1169): outer half
+    kick and respa_inner x (half kick, drift, wrap, bonded forces, half kick)
+    as one differentiable launch, then in torch operations field forces,
+    outer half kick, and the CSVR thermostat of outer step `step` when the
+    RespaMD is coupled."""
     md = model.md
     m, dt, n_in = md.mass, md.dt, md.respa
     dto = n_in * dt
-    v = v + (0.5 * dto / m) * f_field
-    for _ in range(n_in):
-        v = v + (0.5 * dt / m) * f_bond
-        x = torch.remainder(x + dt * v, model.box_f)
-        f_bond = bonded_force(x, model)
-        v = v + (0.5 * dt / m) * f_bond
+    if model.fused_inner:
+        x, v, f_bond = _InnerLoop.apply(x, v, f_field, f_bond, model)
+    else:
+        v = v + (0.5 * dto / m) * f_field
+        for _ in range(n_in):
+            v = v + (0.5 * dt / m) * f_bond
+            x = torch.remainder(x + dt * v, model.box_f)
+            f_bond = bonded_force(x, model)
+            v = v + (0.5 * dt / m) * f_bond
     f_field = field_force(x, chi, model)
     v = v + (0.5 * dto / m) * f_field
     if model.thermo is not None and step is not None:

@@ -576,6 +576,19 @@ int hpf_respa_step_paint(hpf_respa_plan* plan, float* r, float* v, float* f_bond
                          const double* randoms, int* counter, double* state, int* d_err,
                          void* stream);
 
+/* Reverse mode of hpf_respa_step (without barostat): r, v, f_bonded and the
+ * slow forces are the step's INPUTS; gx, gv, gf hold the cotangents of its
+ * outputs r, v, f_bonded and are overwritten with the gradients of the inputs;
+ * gslow (may be NULL) receives the gradient of each slow force (the same for
+ * all).  traj: scratch of float4[respa_inner][bonded beads of the plan], 16-byte
+ * aligned.  The bonded forces' Jacobian is that of hpf_bonded_hvp /
+ * hpf_dihedral_hvp, summed in a fixed order.  A plan whose largest group does
+ * not fit shared memory (hpf_respa_vjp_ok: 0) returns HPF_ERR_NOT_IMPLEMENTED. */
+int hpf_respa_vjp_ok(const hpf_respa_plan* plan, int* ok);
+int hpf_respa_vjp(hpf_respa_plan* plan, const float* r, const float* v, const float* f_bonded,
+                  const float* const* slow_forces, int n_slow, double mass, double dt,
+                  int respa_inner, const double* box, float* gx, float* gv, float* gf,
+                  float* gslow, void* traj, void* stream);
 /* Bonded forces (bonds, angles, dihedrals with CBT) of the plan's topology at
  * positions r, without any integration: f_bonded of every bead in a bonded
  * term is overwritten with its force (other beads untouched), summed in the
