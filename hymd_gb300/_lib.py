@@ -56,6 +56,7 @@ _SIGNATURES = {
     "hpf_c2r": [P, P, P, I, P],
     "hpf_kspace_force": [P, P, P, P, P, P, P],
     "hpf_kspace_sums": [P, P, P, ctypes.POINTER(D), P, P],
+    "hpf_update_field": [P, P, P, I64, ctypes.POINTER(D), P, P, P, P, P, P],
     "hpf_laplacian": [P, P, P, P],
     "hpf_energy_fp64": [P, P, P, I64, ctypes.POINTER(D), P, ctypes.POINTER(D), D, P, P],
     "hpf_readout": [P, P, P, P, I64, P, P],

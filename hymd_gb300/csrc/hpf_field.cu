@@ -1212,6 +1212,41 @@ int hpf_kspace_sums(hpf_ctx* c, const void* phi_fourier, const void* psi_k,
     return HPF_OK;
 }
 
+int hpf_update_field(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n,
+                     const double* type_mass, float* phi, void* phi_fourier, float* force_mesh,
+                     float* v_ext, void* v_k, void* stream) {
+    if (!c || (n > 0 && (!pos || !types)) || !type_mass || !phi || !phi_fourier || !force_mesh ||
+        n < 0 || (v_ext && !v_k))
+        return HPF_ERR_ARG;
+    cudaStream_t st = as_stream(stream);
+    const int T = c->T;
+    TypeScale sc;
+    for (int t = 0; t < T; ++t) sc.s[t] = (float)type_mass[t];
+    const uintptr_t at = reinterpret_cast<uintptr_t>(phi) |
+                         reinterpret_cast<uintptr_t>(phi_fourier) |
+                         reinterpret_cast<uintptr_t>(force_mesh) | reinterpret_cast<uintptr_t>(v_ext);
+    int r;
+    if (spectral_fields_ok(c) && (at & 7) == 0) {
+        if ((r = do_paint(c, pos, types, nullptr, n, T, sc, phi, st, nullptr, false)) != HPF_OK)
+            return r;
+        return spectral_fields(c, sc.s, phi, (float2*)phi_fourier, force_mesh, v_ext, st);
+    }
+    // cuFFT: the k-space pass writes into the context's scratch spectra, which
+    // the inverse transforms may overwrite; only the caller's filtered spectra
+    // are copied
+    if ((r = do_paint(c, pos, types, nullptr, n, T, sc, phi, st)) != HPF_OK) return r;
+    if ((r = exec_r2c(c, phi, c->d_spec_phi, T, st)) != HPF_OK) return r;
+    if ((r = launch_kspace_force(c, c->d_spec_phi, c->d_spec, (float2*)phi_fourier,
+                                 v_ext ? (float2*)v_k : nullptr, nullptr, st)) != HPF_OK)
+        return r;
+    if ((r = exec_c2r(c, c->d_spec, force_mesh, 3 * T, st)) != HPF_OK) return r;
+    HPF_CUDA_TRY(cudaMemcpyAsync(c->d_spec, phi_fourier, sizeof(float2) * (size_t)T * c->Mc,
+                                 cudaMemcpyDeviceToDevice, st));
+    if ((r = exec_c2r(c, c->d_spec, phi, T, st)) != HPF_OK) return r;
+    if (v_ext) return exec_c2r(c, (const float2*)v_k, v_ext, T, st);
+    return HPF_OK;
+}
+
 int hpf_energy_fp64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n,
                     const double* type_mass, const float* charges, const double* type_charges,
                     double elec_factor, double* out, void* stream) {
@@ -1354,13 +1389,23 @@ int hpf_pic_step(hpf_ctx* c, const float* pos, const float* charges, int64_t n,
     sc.s[0] = 1.0f;
     const float four_pi_fac = (float)(4.0 * 3.14159265358979323846 * elec_factor);
     int r;
-    if (c->spec_fused && !phi_q && !psi_k) {
-        // fused passes (no real charge grid or psi spectrum is produced)
-        if ((r = do_paint(c, pos, nullptr, charges, n, 1, sc, c->d_grid, st, nullptr, false)) !=
-            HPF_OK)
+    // the fused passes write the caller's grids and spectrum themselves, as
+    // float2
+    const uintptr_t at = reinterpret_cast<uintptr_t>(phi_q) | reinterpret_cast<uintptr_t>(psi) |
+                         reinterpret_cast<uintptr_t>(elec_field) |
+                         reinterpret_cast<uintptr_t>(psi_k);
+    if (c->spec_fused && (at & 7) == 0) {
+        if ((r = do_paint(c, pos, nullptr, charges, n, 1, sc, phi_q ? phi_q : c->d_grid, st, nullptr,
+                          phi_q != nullptr)) != HPF_OK)
             return r;
-        if ((r = spectral_pic(c, main_bufs(c), four_pi_fac, psi != nullptr, sums, st)) != HPF_OK)
+        const PicOut o{psi, elec_field, (float2*)psi_k};
+        if ((r = spectral_pic(c, main_bufs(c), four_pi_fac, psi != nullptr, sums, st, phi_q, true,
+                              o)) != HPF_OK)
             return r;
+        if (n > 0)
+            return launch_readout(c, elec_field ? elec_field : c->d_grid + c->M, pos, nullptr,
+                                  charges, n, 1, elec_forces, kick, st);
+        return HPF_OK;
     } else {
         float* rho = phi_q ? phi_q : c->d_grid;
         if ((r = do_paint(c, pos, nullptr, charges, n, 1, sc, rho, st)) != HPF_OK) return r;

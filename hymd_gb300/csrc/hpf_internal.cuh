@@ -115,6 +115,13 @@ struct SpecBufs {
     double* ws;
 };
 
+// Where the charge chain leaves psi, E[3][M] and psi's half spectrum, when not
+// in its own grids.
+struct PicOut {
+    float *psi, *E;
+    float2* psi_k;
+};
+
 // Paint deposits are integers in units of 2^-24 of a particle's weight (a
 // charge of up to 2^7 e keeps a deposit inside int32).
 constexpr float kFixScale = 16777216.0f;          // 2^24
@@ -142,7 +149,12 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
 // charge accumulator; filter = false drops H(k) from the Poisson map (the GPE
 // solve's psi = scale (q + pol) / k^2).
 int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi, double* sums,
-                 cudaStream_t st, const float* real_in = nullptr, bool filter = true);
+                 cudaStream_t st, const float* real_in = nullptr, bool filter = true,
+                 const PicOut& o = PicOut{nullptr, nullptr, nullptr});
+// painted accumulators -> the grids and spectra of update_field
+bool spectral_fields_ok(const hpf_ctx* c);
+int spectral_fields(hpf_ctx* c, const float* type_scale, float* phi, float2* phi_k, float* force,
+                    float* vext, cudaStream_t st);
 // FP64 energy sums in double-float arithmetic (hpf_energy.cu): whether they
 // apply, setup on first use, painted accumulators (G grids) -> out[32].
 bool energy_df_ok(const hpf_ctx* c);

@@ -239,12 +239,15 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
 // of two columns per type (-i g_x v_t and v_t, v_t from the k-space map
 // applied in place to the transformed densities), whose second step writes
 // the output spectra.  Tile layout [grid][x][w], grids g.ts apart.
-template <int N>
+// FIELDS (the drop-in update_field): the filtered densities are wanted too,
+// as spectra (phi_k, half spectra in natural order) and as a third column per
+// type (for their real grids).
+template <int N, bool FIELDS = false>
 __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_kspace(const float2* __restrict__ phi, float2* __restrict__ force, SpecGeom g, int T,
                   const BoxState* __restrict__ bs, const Functional* __restrict__ fun,
                   const float2* __restrict__ tw, double* sums, double* partials,
-                  unsigned int* ticket) {
+                  unsigned int* ticket, float2* __restrict__ phi_k) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
     __shared__ float sQ[kSpecMaxT * kSpecMaxT], sb[kSpecMaxT];
@@ -252,8 +255,10 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     const int W = g.W, ws = g.ws, TS = g.ts;
     const int64_t plane = (int64_t)g.n1 * g.nzc;  // stride of x in a half spectrum
     const int j0 = blockIdx.x * W;
-    float2* in = sm;            // [T][Nx][W]
-    float2* out = sm + T * TS;  // [2T][Nx][W]
+    constexpr int NO = FIELDS ? 3 : 2;  // output columns per type
+    float2* in = sm;                    // [T][Nx][W]
+    float2* flt = sm + T * TS;          // FIELDS: filtered densities, [T][Nx][W]
+    float2* out = sm + (FIELDS ? 2 : 1) * T * TS;  // [NO T][Nx][W]
     for (int e = threadIdx.x; e < T * T; e += blockDim.x)
         sQ[(e / T) * kSpecMaxT + e % T] = fun->Q[e];
     for (int e = threadIdx.x; e < T; e += blockDim.x) sb[e] = fun->b[e];
@@ -264,7 +269,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     const float invM = (float)bs->inv_M * bs->inv_dV;
     const float s2h = fun->sigma2_half;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const int cin = T * W, cout = 2 * T * W;
+    const int cin = T * W, cout = NO * T * W;
     const float inv_cin = 1.0f / (float)cin, inv_cout = 1.0f / (float)cout;
     {
         constexpr int N1 = split1(N), N2 = N / N1;
@@ -302,6 +307,14 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                 float2 ph[TT];
 #pragma unroll
                 for (int jj = 0; jj < TT; ++jj) ph[jj] = in[jj * TS + p * W + w];
+                if (FIELDS) {
+#pragma unroll
+                    for (int jj = 0; jj < TT; ++jj) {
+                        const float2 f = make_float2(hm * ph[jj].x, hm * ph[jj].y);
+                        flt[jj * TS + p * W + w] = f;
+                        phi_k[(int64_t)jj * g.Mc + ix * plane + j0 + w] = f;
+                    }
+                }
                 float qq = 0.0f;
 #pragma unroll
                 for (int tt = 0; tt < TT; ++tt) {
@@ -337,17 +350,17 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
             default: map(IntC<8>()); break;
         }
         __syncthreads();
-        // inverse x transforms, step 1; item (grid 2 to + e, w, n2): e = 0
+        // inverse x transforms, step 1; item (grid NO to + e, w, n2): e = 0
         // -i g_x v_to (the x force), e = 1 v_to itself (the y and z forces,
         // -i g_y v and -i g_z v, are formed from it in pass C: g_y and g_z
-        // do not vary along x)
+        // do not vary along x), e = 2 the filtered density
         const int items = cout * N2;
         for (int it = threadIdx.x; it < items; it += blockDim.x) {
             const int n2 = N2 == 1 ? 0 : div_inv(it, cout, inv_cout);
             const int c = it - n2 * cout;
             const int gq = c >> ws, w = c & (W - 1);
-            const int to = gq >> 1, e = gq & 1;
-            const float2* vt = in + to * TS + w;
+            const int to = gq / NO, e = gq - to * NO;
+            const float2* vt = (FIELDS && e == 2 ? flt : in) + to * TS + w;
             float2 a[N1];
 #pragma unroll
             for (int i = 0; i < N1; ++i) {
@@ -397,7 +410,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                       const BoxState* __restrict__ bs, const Functional* __restrict__ fun,
                       float four_pi_fac, const float2* __restrict__ tw,
                       double* sums, double* partials, unsigned int* ticket, int filter,
-                      int by_volume) {
+                      int by_volume, float2* __restrict__ psi_k) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
     __shared__ ColInfo col[16];
@@ -447,6 +460,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                 const float2 rq = make_float2(r.x * invM, r.y * invM);
                 const float sc = four_pi_fac * Hk / k2;
                 const float2 v = make_float2(rq.x * sc, rq.y * sc);
+                if (psi_k && e) psi_k[ix * plane + j0 + w] = v;
                 if (sums && e == 0)
                     acc[0] = fmaf(ci.wk, fmaf(rq.x, v.x, rq.y * v.y), acc[0]);
                 const float gx = ix == N / 2 ? 0.0f : kx;
@@ -492,15 +506,20 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
 // the packing is computed in the z transform's first step (rows handled by
 // one warp each, since X[m] and X[h-m] are overwritten in place) and its
 // second step writes the real plane.
-// Output grid gi (density: 3 t + d; PIC: psi, E_x, E_y, E_z) comes from
-// pass B's grid src: -i g_x v (x force) as is, v times -i g_y (a function
-// of the row ky) or -i g_z (of the column kz) for the y and z forces, v as
-// is for psi.
+// Output grid gi comes from pass B's grid src: -i g_x v (x force) as is, v
+// times -i g_y (a function of the row ky) or -i g_z (of the column kz) for the
+// y and z forces, v (psi, the external potential) and the filtered density as
+// they are.
+//   kDensity: gi = 3 t + d, force grids of `grid`
+//   kPic:     gi = 0 psi (`aux`), 1..3 E_d (`grid`)
+//   kFields:  gi < 3 T as kDensity, then T filtered densities (`aux`), then T
+//             external potentials (`aux2`)
+enum SpecOut { kDensity = 0, kPic = 1, kFields = 2 };
 template <int NY, int HZ>
 __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_inv(const float2* __restrict__ spec, float* __restrict__ grid, SpecGeom g,
                const BoxState* __restrict__ bs, const float2* __restrict__ tw, int first,
-               int pic) {
+               int mode, int T, float* aux, float* aux2) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
     constexpr int Ny = NY, H = HZ, Nzc = H + 1, Ls = plane_ls(H), PN = plane_n2(H);
@@ -511,17 +530,27 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     auto zs = [](int e) { return PN > 1 ? e + e / PN : e; };
     auto row0 = [](int r) { return plane_row<NY, HZ>(r); };
     int src, mul;  // mul: 0 none, 1 -i g_y, 2 -i g_z
-    if (pic) {
+    float* base = grid;
+    int oi = gi;
+    if (mode == kPic) {
         src = gi == 1 ? 0 : 1;
         mul = gi == 2 ? 1 : (gi == 3 ? 2 : 0);
+        if (gi == 0) base = aux;
+        else oi = gi - 1;
+    } else if (mode == kFields && gi >= 3 * T) {
+        const bool pot = gi >= 4 * T;
+        oi = gi - (pot ? 4 : 3) * T;
+        base = pot ? aux2 : aux;
+        src = 3 * oi + (pot ? 1 : 2);
+        mul = 0;
     } else {
         const int t = gi / 3, d = gi - 3 * t;
-        src = 2 * t + (d > 0);
+        src = (mode == kFields ? 3 : 2) * t + (d > 0);
         mul = d;
     }
     const float kf1 = bs->kf[1], kf2 = bs->kf[2];
     const float2* in = spec + (int64_t)src * g.Mc + (int64_t)x * Ny * Nzc;
-    float2* out = reinterpret_cast<float2*>(grid + ((int64_t)gi * g.n0 + x) * Ny * (2 * H));
+    float2* out = reinterpret_cast<float2*>(base + ((int64_t)oi * g.n0 + x) * Ny * (2 * H));
     constexpr float inv_rows = 1.0f / (float)Ny, inv_cols = 1.0f / (float)Nzc;
     {
         // y: rows left at FftIdx positions of y
@@ -597,16 +626,16 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
 template <class F>
 int with_kspace(int nx, F f) {
     switch (nx) {
-        case 8: return f(k_spec_kspace<8>, k_spec_kspace_pic<8>);
-        case 16: return f(k_spec_kspace<16>, k_spec_kspace_pic<16>);
-        case 32: return f(k_spec_kspace<32>, k_spec_kspace_pic<32>);
-        case 64: return f(k_spec_kspace<64>, k_spec_kspace_pic<64>);
-        case 128: return f(k_spec_kspace<128>, k_spec_kspace_pic<128>);
-        case 256: return f(k_spec_kspace<256>, k_spec_kspace_pic<256>);
-        case 24: return f(k_spec_kspace<24>, k_spec_kspace_pic<24>);
-        case 48: return f(k_spec_kspace<48>, k_spec_kspace_pic<48>);
-        case 96: return f(k_spec_kspace<96>, k_spec_kspace_pic<96>);
-        case 192: return f(k_spec_kspace<192>, k_spec_kspace_pic<192>);
+        case 8: return f(k_spec_kspace<8>, k_spec_kspace_pic<8>, k_spec_kspace<8, true>);
+        case 16: return f(k_spec_kspace<16>, k_spec_kspace_pic<16>, k_spec_kspace<16, true>);
+        case 32: return f(k_spec_kspace<32>, k_spec_kspace_pic<32>, k_spec_kspace<32, true>);
+        case 64: return f(k_spec_kspace<64>, k_spec_kspace_pic<64>, k_spec_kspace<64, true>);
+        case 128: return f(k_spec_kspace<128>, k_spec_kspace_pic<128>, k_spec_kspace<128, true>);
+        case 256: return f(k_spec_kspace<256>, k_spec_kspace_pic<256>, k_spec_kspace<256, true>);
+        case 24: return f(k_spec_kspace<24>, k_spec_kspace_pic<24>, k_spec_kspace<24, true>);
+        case 48: return f(k_spec_kspace<48>, k_spec_kspace_pic<48>, k_spec_kspace<48, true>);
+        case 96: return f(k_spec_kspace<96>, k_spec_kspace_pic<96>, k_spec_kspace<96, true>);
+        case 192: return f(k_spec_kspace<192>, k_spec_kspace_pic<192>, k_spec_kspace<192, true>);
         default: return HPF_ERR_ARG;
     }
 }
@@ -666,6 +695,11 @@ size_t tile_smem(const hpf_ctx* c, int W, bool pic = false) {
     return sizeof(float2) * (size_t)blocks * (c->n0 * W + tile_pad(W));
 }
 
+// a tile with the filtered densities: T in, T filtered, 3T out
+size_t fields_smem(const hpf_ctx* c, int W) {
+    return sizeof(float2) * (size_t)(5 * c->T) * (c->n0 * W + tile_pad(W));
+}
+
 // The widest tile of W in {16, 8, 4} columns that divides n1, fits the
 // shared-memory budget and leaves a tile for every SM (4 when none does).
 // The charge pass takes it for itself: with one grid in, narrower tiles
@@ -683,7 +717,7 @@ int widest_tile(const hpf_ctx* c, bool pic) {
 // Whether the fused passes apply to this context's mesh and type count.
 bool spectral_eligible(const hpf_ctx* c) {
     if (c->T > kSpecMaxT) return false;
-    if (with_kspace(c->n0, [](auto, auto) { return HPF_OK; }) != HPF_OK) return false;
+    if (with_kspace(c->n0, [](auto, auto, auto) { return HPF_OK; }) != HPF_OK) return false;
     if (plane_smem(c) > kSpecMaxSmem) return false;
     if (with_planes(c->n1, c->n2 / 2, [](auto, auto, auto) { return HPF_OK; }) != HPF_OK) return false;
     return tile_smem(c, 4) <= kSpecTileSmem;
@@ -748,10 +782,12 @@ int spectral_setup(hpf_ctx* c) {
                        ? HPF_ERR_CUDA
                        : HPF_OK;
         }) != HPF_OK ||
-        with_kspace(c->n0, [&](auto kd, auto kp) {
+        with_kspace(c->n0, [&](auto kd, auto kp, auto kf) {
             return (cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, ts) !=
                         cudaSuccess ||
                     cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, ts) !=
+                        cudaSuccess ||
+                    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, ts) !=
                         cudaSuccess)
                        ? HPF_ERR_CUDA
                        : HPF_OK;
@@ -782,9 +818,9 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
     if (join) HPF_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
     double* part = c->d_spec_ws;
     unsigned int* tick = reinterpret_cast<unsigned int*>(c->d_spec_ws + 4 * (size_t)c->spec_max_tiles);
-    int r = with_kspace(c->n0, [&](auto kd, auto) {
+    int r = with_kspace(c->n0, [&](auto kd, auto, auto) {
         return launch_pdl(kd, c->spec_tiles, kSpecThreads, ts, st, c->d_spec_phi, c->d_spec, g,
-                          c->T, c->d_box, c->d_fun, c->d_tw, sums, part, tick) == cudaSuccess
+                          c->T, c->d_box, c->d_fun, c->d_tw, sums, part, tick, nullptr) == cudaSuccess
                    ? HPF_OK
                    : HPF_ERR_CUDA;
     });
@@ -792,7 +828,8 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
     HPF_LAUNCH_CHECK();
     if (with_planes(c->n1, c->n2 / 2, [&](auto, auto ki, auto) {
             return launch_pdl(ki, dim3(c->n0, 3 * c->T), kSpecThreads, ps, st, c->d_spec,
-                              c->d_grid, g, c->d_box, c->d_tw, 0, 0) == cudaSuccess
+                              c->d_grid, g, c->d_box, c->d_tw, 0, (int)kDensity, c->T, nullptr,
+                              nullptr) == cudaSuccess
                        ? HPF_OK
                        : HPF_ERR_CUDA;
         }) != HPF_OK)
@@ -800,11 +837,52 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
     return HPF_OK;
 }
 
-// charge accumulator (slot T, painted), or the real grid real_in -> psi
-// (grid 0, when want_psi) and E_d (grids 1..3) in b.grid; sums[0] as
-// k_kspace_pic's when non-null.
+// The drop-in update_field from painted accumulators: filtered densities phi
+// [T][M], their half spectra phi_k [T][Mc], the force mesh [T][3][M] and, when
+// vext is given, the filtered external potentials [T][M].
+int spectral_fields(hpf_ctx* c, const float* type_scale, float* phi, float2* phi_k, float* force,
+                    float* vext, cudaStream_t st) {
+    int W = 16;
+    const int64_t cols = (int64_t)c->n1 * (c->n2 / 2 + 1);
+    while (W > 4 && (c->n1 % W != 0 || fields_smem(c, W) > kSpecTileSmem || cols / W < 152)) W >>= 1;
+    const SpecGeom g = spec_geom(c, W);
+    SpecScale sc;
+    for (int t = 0; t < c->T; ++t) sc.s[t] = type_scale[t];
+    const int ps = (int)plane_smem(c), ts = (int)fields_smem(c, W);
+    int r = with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto) {
+        return launch_pdl(kf, dim3(c->n0, c->T), kSpecThreads, ps, st, c->d_acc, c->d_spec_phi, g,
+                          sc, c->d_tw, nullptr) == cudaSuccess
+                   ? HPF_OK
+                   : HPF_ERR_CUDA;
+    });
+    if (r != HPF_OK) return r;
+    r = with_kspace(c->n0, [&](auto, auto, auto kf) {
+        return launch_pdl(kf, dim3((unsigned)(cols / W)), kSpecThreads, ts, st, c->d_spec_phi,
+                          c->d_spec, g, c->T, c->d_box, c->d_fun, c->d_tw, nullptr, nullptr,
+                          nullptr, phi_k) == cudaSuccess
+                   ? HPF_OK
+                   : HPF_ERR_CUDA;
+    });
+    if (r != HPF_OK) return r;
+    return with_planes(c->n1, c->n2 / 2, [&](auto, auto ki, auto) {
+        return launch_pdl(ki, dim3(c->n0, (vext ? 5 : 4) * c->T), kSpecThreads, ps, st, c->d_spec,
+                          force, g, c->d_box, c->d_tw, 0, (int)kFields, c->T, phi, vext) ==
+                       cudaSuccess
+                   ? HPF_OK
+                   : HPF_ERR_CUDA;
+    });
+}
+
+bool spectral_fields_ok(const hpf_ctx* c) {
+    return c->spec_ok && c->spec_fused && fields_smem(c, 4) <= kSpecTileSmem;
+}
+
+// charge accumulator (slot T, painted), or the real grid real_in -> psi (when
+// want_psi) and E_d, in o's grids or by default in b.grid's grid 0 and 1..3;
+// psi's half spectrum into o.psi_k when given; sums[0] as k_kspace_pic's when
+// non-null.
 int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi, double* sums,
-                 cudaStream_t st, const float* real_in, bool filter) {
+                 cudaStream_t st, const float* real_in, bool filter, const PicOut& o) {
     const SpecGeom g = spec_geom(c, c->spec_W_pic);
     SpecScale sc;
     sc.s[0] = 1.0f;
@@ -821,10 +899,10 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
         return HPF_ERR_CUDA;
     double* part = b.ws;
     unsigned int* tick = reinterpret_cast<unsigned int*>(b.ws + 4 * (size_t)c->spec_max_tiles);
-    int r = with_kspace(c->n0, [&](auto, auto kp) {
+    int r = with_kspace(c->n0, [&](auto, auto kp, auto) {
         return launch_pdl(kp, c->spec_tiles_pic, kSpecThreads, ts, st, b.spec_phi, b.spec, g,
                           c->d_box, c->d_fun, four_pi_fac, c->d_tw, sums, part, tick,
-                          filter ? 1 : 0, real_in ? 0 : 1) == cudaSuccess
+                          filter ? 1 : 0, real_in ? 0 : 1, o.psi_k) == cudaSuccess
                    ? HPF_OK
                    : HPF_ERR_CUDA;
     });
@@ -832,8 +910,9 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
     HPF_LAUNCH_CHECK();
     const int first = want_psi ? 0 : 1;
     if (with_planes(c->n1, c->n2 / 2, [&](auto, auto ki, auto) {
-            return launch_pdl(ki, dim3(c->n0, 4 - first), kSpecThreads, ps, st, b.spec, b.grid,
-                              g, c->d_box, c->d_tw, first, 1) == cudaSuccess
+            return launch_pdl(ki, dim3(c->n0, 4 - first), kSpecThreads, ps, st, b.spec,
+                              o.E ? o.E : b.grid + c->M, g, c->d_box, c->d_tw, first, (int)kPic,
+                              c->T, o.psi ? o.psi : b.grid, nullptr) == cudaSuccess
                        ? HPF_OK
                        : HPF_ERR_CUDA;
         }) != HPF_OK)

@@ -48,8 +48,6 @@ class ParticleMesh:
         self.box_state_ptr = st.value
         self._functional = None
         self.ws = _lib.new_workspace(self.device)
-        self.spec_raw = self.complex_field(self.n_types)
-        self.spec_force = self.complex_field(3 * self.n_types)
 
     # -- allocation helpers -------------------------------------------------
     def real_field(self, *lead):
@@ -293,16 +291,13 @@ def update_field(phi, phi_laplacian, phi_transfer, layouts, force_mesh, hamilton
     pm.set_functional(hamiltonian)
     st = _lib.stream_ptr()
     masses = _lib.dvec(_masses(m, T))
-    _lib.call("hpf_paint", pm._h, _lib.ptr(pos), _lib.ptr(typ), n, masses, _lib.ptr(phi_all), st)
-    _lib.call("hpf_r2c", pm._h, _lib.ptr(phi_all), _lib.ptr(pm.spec_raw), T, st)
-    v_k = pm.complex_field(T) if compute_potential else None
-    _lib.call("hpf_kspace_force", pm._h, _lib.ptr(pm.spec_raw), _lib.ptr(pm.spec_force),
-              _lib.ptr(phif_all), _lib.ptr(v_k), None, st)
-    _lib.call("hpf_c2r", pm._h, _lib.ptr(pm.spec_force), _lib.ptr(force_all), 3 * T, st)
-    _lib.call("hpf_c2r", pm._h, _lib.ptr(phif_all), _lib.ptr(phi_all), T, st)
+    vext_all = v_k = None
     if compute_potential:
         vext_all = _stack_base(v_ext, (T,), torch.float32, "v_ext")
-        _lib.call("hpf_c2r", pm._h, _lib.ptr(v_k), _lib.ptr(vext_all), T, st)
+        v_k = pm.complex_field(T)
+    _lib.call("hpf_update_field", pm._h, _lib.ptr(pos), _lib.ptr(typ), n, masses,
+              _lib.ptr(phi_all), _lib.ptr(phif_all), _lib.ptr(force_all), _lib.ptr(vext_all),
+              _lib.ptr(v_k), st)
     pm.last_types = typ
 
 

@@ -320,6 +320,14 @@ int hpf_laplacian(hpf_ctx* ctx, const void* phi_fourier, float* lap_out, void* s
 int hpf_readout(hpf_ctx* ctx, const float* force_mesh, const float* pos,
                 const int32_t* types, int64_t n, float* force, void* stream);
 
+/* update_field (hymd/field.py:428-616) with the grids it leaves behind: phi
+ * float[T][M] the filtered densities, phi_fourier float2[T][Mc] their half
+ * spectra (H r2c(phi), normalised by 1/M), force_mesh float[T][3][M] and, when
+ * v_ext is given, the filtered external potentials float[T][M]; v_k (with
+ * v_ext) is scratch float2[T][Mc]. */
+int hpf_update_field(hpf_ctx* ctx, const float* pos, const int32_t* types, int64_t n,
+                     const double* type_mass, float* phi, void* phi_fourier, float* force_mesh,
+                     float* v_ext, void* v_k, void* stream);
 /* ---- whole field evaluation ----------------------------------------------
  * update_field + compute_field_force (field.py:428-616, 152-200) without the
  * real-space intermediates: paint -> r2c -> fused k-space -> c2r(3T) ->
