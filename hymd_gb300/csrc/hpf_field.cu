@@ -1492,9 +1492,8 @@ int hpf_field_pic_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
     float* pos_w = painted && pos_scale ? pos : nullptr;
     const double* rscale = painted ? pos_scale : nullptr;
     cudaStream_t st = as_stream(stream);
-    // rRESPA sums still running beside this call: waited for before the
-    // k-space pass, the first kernel here that reads the box; deposits yet to
-    // be made read it too, and with charges both chains follow them
+    // rRESPA sums still running beside this call, joined before the k-space
+    // pass; at once where the deposits are still to be made or both chains run
     cudaEvent_t join = c->pending;
     c->pending = nullptr;
     if (join && (!painted || charges)) {

@@ -99,9 +99,9 @@ struct hpf_ctx {
     double* pic_spec_ws;
     cudaStream_t pic_stream;
     cudaEvent_t pic_fork, pic_join;
-    // the rRESPA sums (and the barostat's box update) still running on their
-    // plan's second stream (hpf_respa_plan_defer): the field step waits for
-    // this event before its k-space pass, then forgets it.  Owned by the plan.
+    // the rRESPA sums still running on their plan's second stream
+    // (hpf_respa_plan_defer): the field step waits for this event before its
+    // k-space pass, then forgets it.  Owned by the plan.
     cudaEvent_t pending;
 };
 

@@ -1487,7 +1487,7 @@ int respa_run(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
     }
     if (split) HPF_CUDA_TRY(cudaStreamWaitEvent(st, p->free_join, 0));
     if (rc != HPF_OK) return rc;
-    if (out && pf && p->defer) {
+    if (out && pf && p->defer && !baro) {
         // the sums (one block, a latency chain) beside the field step's first
         // pass instead of before it
         HPF_CUDA_TRY(cudaEventRecord(p->sums_fork, st));

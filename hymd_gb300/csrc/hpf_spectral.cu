@@ -116,15 +116,12 @@ __device__ __forceinline__ int plane_row(int r) {
 // the half spectrum X[0..h] fused into the first step of the y transform;
 // the y transform's second step writes the spectrum plane.
 // blockIdx.y: the grid (type) of acc and spec; sc.s[that grid] scales it.
-// The accumulators become painted weights per cell here; the division by the
-// cell volume is pass B's, so that this pass does not need the box and can
-// run while a barostat still updates it.
 // FIX = false: the input is a real grid (fin, float[grids][M]) scaled by
 // sc.s[grid] alone, read and left as it is (the accumulators are not used).
 template <int NY, int HZ, bool FIX = true>
 __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_fwd(unsigned long long* __restrict__ acc, float2* __restrict__ spec, SpecGeom g,
-               SpecScale sc, const float2* __restrict__ tw,
+               SpecScale sc, const BoxState* __restrict__ bs, const float2* __restrict__ tw,
                const float* __restrict__ fin = nullptr) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
@@ -135,7 +132,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto zs = [](int e) { return PN > 1 ? e + e / PN : e; };
     auto row0 = [](int r) { return plane_row<NY, HZ>(r); };
-    const float s = FIX ? sc.s[t] * kFixInv : sc.s[t];
+    const float s = FIX ? sc.s[t] * bs->inv_dV * kFixInv : sc.s[t];
     ulonglong2* a =
         FIX ? reinterpret_cast<ulonglong2*>(acc + (int64_t)t * g.M + (int64_t)x * Ny * (2 * H))
             : nullptr;
@@ -265,8 +262,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     tile_columns(col, g, j0, bs);
     using fx = Idx<N>;
     const float kf0 = bs->kf[0];
-    // 1 / M of the unnormalised transform, and the weights' 1 / dV
-    const float invM = (float)bs->inv_M * bs->inv_dV;
+    const float invM = (float)bs->inv_M;
     const float s2h = fun->sigma2_half;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     const int cin = T * W, cout = NO * T * W;
@@ -410,7 +406,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                       const BoxState* __restrict__ bs, const Functional* __restrict__ fun,
                       float four_pi_fac, const float2* __restrict__ tw,
                       double* sums, double* partials, unsigned int* ticket, int filter,
-                      int by_volume, float2* __restrict__ psi_k) {
+                      float2* __restrict__ psi_k) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
     __shared__ ColInfo col[16];
@@ -422,9 +418,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     tile_columns(col, g, j0, bs);
     using fx = Idx<N>;
     const float kf0 = bs->kf[0];
-    // by_volume: the input spectrum is that of weights per cell (a real grid
-    // holds densities)
-    const float invM = by_volume ? (float)bs->inv_M * bs->inv_dV : (float)bs->inv_M;
+    const float invM = (float)bs->inv_M;
     const float s2h = fun->sigma2_half;
     float acc[1] = {0.0f};
     const int cout = 2 * W;
@@ -810,7 +804,7 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
     const int ps = (int)plane_smem(c), ts = (int)tile_smem(c, g.W);
     if (with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto) {
             return launch_pdl(kf, dim3(c->n0, c->T), kSpecThreads, ps, st, c->d_acc,
-                              c->d_spec_phi, g, sc, c->d_tw, nullptr) == cudaSuccess
+                              c->d_spec_phi, g, sc, c->d_box, c->d_tw, nullptr) == cudaSuccess
                        ? HPF_OK
                        : HPF_ERR_CUDA;
         }) != HPF_OK)
@@ -851,7 +845,7 @@ int spectral_fields(hpf_ctx* c, const float* type_scale, float* phi, float2* phi
     const int ps = (int)plane_smem(c), ts = (int)fields_smem(c, W);
     int r = with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto) {
         return launch_pdl(kf, dim3(c->n0, c->T), kSpecThreads, ps, st, c->d_acc, c->d_spec_phi, g,
-                          sc, c->d_tw, nullptr) == cudaSuccess
+                          sc, c->d_box, c->d_tw, nullptr) == cudaSuccess
                    ? HPF_OK
                    : HPF_ERR_CUDA;
     });
@@ -890,10 +884,10 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
     if (with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto kr) {
             const cudaError_t e =
                 real_in ? launch_pdl(kr, dim3(c->n0, 1), kSpecThreads, ps, st, nullptr,
-                                     b.spec_phi, g, sc, c->d_tw, real_in)
+                                     b.spec_phi, g, sc, c->d_box, c->d_tw, real_in)
                         : launch_pdl(kf, dim3(c->n0, 1), kSpecThreads, ps, st,
                                      c->d_acc + (int64_t)c->T * c->M, b.spec_phi, g, sc,
-                                     c->d_tw, nullptr);
+                                     c->d_box, c->d_tw, nullptr);
             return e == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
         }) != HPF_OK)
         return HPF_ERR_CUDA;
@@ -902,7 +896,7 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
     int r = with_kspace(c->n0, [&](auto, auto kp, auto) {
         return launch_pdl(kp, c->spec_tiles_pic, kSpecThreads, ts, st, b.spec_phi, b.spec, g,
                           c->d_box, c->d_fun, four_pi_fac, c->d_tw, sums, part, tick,
-                          filter ? 1 : 0, real_in ? 0 : 1, o.psi_k) == cudaSuccess
+                          filter ? 1 : 0, o.psi_k) == cudaSuccess
                    ? HPF_OK
                    : HPF_ERR_CUDA;
     });

@@ -767,14 +767,14 @@ class RespaMD:
 
     @property
     def _defer_sums(self):
-        """step() may leave the inner loop's sums and box update to run beside
-        the field step's first pass, which joins them.  Measured on GB300, us a
-        step in line / beside: 10k melt 41.0 / 37.0, 162k membrane (NPT)
-        105.7 / 101.  With charges the charge chain already fills that gap and
-        the extra branch costs (500k peptides 279 / 297, 60k 135 / 132, 12k
-        94 / 94), so there the sums stay in line; so they do in a subclass
-        with a second half of its own."""
-        return (self._paint_fused and self.charges is None
+        """step() may leave the inner loop's sums to run beside the field
+        step's first pass, which joins them.  Measured on GB300, us a step in
+        line / beside: 10k melt 42.9 / 39.2.  A barostat's box update has to
+        come before that pass.  With charges the charge chain already fills
+        the gap and the extra branch costs (500k peptides 273 / 287, 60k 130 /
+        128, 12k 97 / 96), so there the sums stay in line; so they do in a
+        subclass with a second half of its own."""
+        return (self._paint_fused and self.charges is None and self.baro_args is None
                 and type(self)._outer_rest is RespaMD._outer_rest)
 
     def _inner_fused(self, st, defer=False):

@@ -481,11 +481,11 @@ int hpf_respa_plan_permute(hpf_respa_plan* plan, const int32_t* inv, int64_t n,
 int hpf_respa_plan_counts(const hpf_respa_plan* plan, int64_t* n_bonded, int64_t* n_free);
 int hpf_respa_plan_info(const hpf_respa_plan* plan, int* n_mol_blocks, int* n_free,
                         int* max_block_beads);
-/* on = 1: hpf_respa_step_paint leaves its sums (out) and the barostat's update
- * (box, state, counter) running beside the calls that follow on `stream`, and
- * the next hpf_field_pic_step on its field_ctx, which must follow on the same
- * stream, waits for them; on = 0 (the default): they are complete in stream
- * order when the call returns. */
+/* on = 1: hpf_respa_step_paint without a barostat leaves its sums (out) running
+ * beside the calls that follow on `stream`, and the next hpf_field_pic_step on
+ * its field_ctx, which must follow on the same stream, waits for them; on = 0
+ * (the default), and always with a barostat: complete in stream order when the
+ * call returns. */
 int hpf_respa_plan_defer(hpf_respa_plan* plan, int on);
 /* hpf_respa_step (the launch itself) is declared after the barostat
  * arguments below. */
