@@ -666,6 +666,118 @@ __global__ void k_adjoint_sums(const float2* __restrict__ spec, int64_t Mc, KGeo
     grid_reduce_store_f<P + 1, kThreads>(acc, partials, ticket, out);
 }
 
+// The quadratic functional from its parameters on the device (chi as float or
+// double; neither: no chi), so that fitting chi needs no copy to the host and
+// no synchronisation: Q_ij = 1/(kappa rho0) + (chi_ij + chi_ji)/(2 rho0) off
+// the diagonal, b = -a/(kappa rho0), c = a^2/(2 kappa rho0), in FP64.
+__global__ void k_functional_chi(Functional* fun, int T, const float* __restrict__ chi_f,
+                                 const double* __restrict__ chi_d, double kappa, double rho0,
+                                 double a, double sigma) {
+    const double inc = 1.0 / (kappa * rho0);
+    for (int e = threadIdx.x; e < T * T; e += blockDim.x) {
+        const int i = e / T, j = e - i * T;
+        double q = inc;
+        if (i != j && (chi_f || chi_d)) {
+            const double x = chi_d ? chi_d[e] : (double)chi_f[e];
+            const double y = chi_d ? chi_d[j * T + i] : (double)chi_f[j * T + i];
+            q += 0.5 * (x + y) / rho0;
+        }
+        fun->Qd[e] = q;
+        fun->Q[e] = (float)q;
+    }
+    for (int i = threadIdx.x; i < T; i += blockDim.x) {
+        fun->bd[i] = -a * inc;
+        fun->b[i] = (float)(-a * inc);
+    }
+    if (threadIdx.x == 0) {
+        fun->c = 0.5 * a * a * inc;
+        fun->sigma2_half_d = 0.5 * sigma * sigma;
+        fun->sigma2_half = (float)(0.5 * sigma * sigma);
+    }
+}
+
+// ---------------------------------------------------------- z profile ---
+// Per-type number density along z with linear binning onto bin centres
+// (periodic).  Weights are integers in units of 2^-24 summed in int64, in
+// shared memory where the bins fit (else in global memory), so the profile
+// does not depend on the order of the beads; the last block converts it.
+// scratch: zeroed uint64[T n_bins + 2] (bins, ticket, non-finite flag).
+struct ZBin {
+    int i0, i1;
+    float f;
+    bool ok;
+};
+__device__ __forceinline__ ZBin z_bin(float z, float scale, int nb) {
+    const float s = z * scale - 0.5f;
+    const float fl = floorf(s);
+    ZBin b;
+    b.ok = isfinite(s);
+    b.f = s - fl;
+    int i = b.ok ? (int)fmodf(fl, (float)nb) : 0;
+    if (i < 0) i += nb;
+    b.i0 = i;
+    b.i1 = i + 1 == nb ? 0 : i + 1;
+    return b;
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_z_profile(const float* __restrict__ x, const int32_t* __restrict__ types, int64_t n, int T,
+            int nb, float scale, float inv_vol, unsigned long long* __restrict__ scratch,
+            float* __restrict__ out, int in_shared) {
+    extern __shared__ unsigned long long zb[];
+    __shared__ bool is_last;
+    const int bins = T * nb;
+    unsigned long long* h = in_shared ? zb : scratch;
+    if (in_shared) {
+        for (int i = threadIdx.x; i < bins; i += kThreads) zb[i] = 0ull;
+        __syncthreads();
+    }
+    for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * kThreads) {
+        const ZBin b = z_bin(x[3 * i + 2], scale, nb);
+        const int t = types[i];
+        if (!b.ok || t < 0 || t >= T) {
+            atomicOr(scratch + bins + 1, 1ull);
+            continue;
+        }
+        atomicAdd(h + t * nb + b.i0,
+                  (unsigned long long)(long long)__float2int_rn((1.0f - b.f) * kFixScale));
+        atomicAdd(h + t * nb + b.i1, (unsigned long long)(long long)__float2int_rn(b.f * kFixScale));
+    }
+    __syncthreads();
+    if (in_shared)
+        for (int i = threadIdx.x; i < bins; i += kThreads)
+            if (zb[i]) atomicAdd(scratch + i, zb[i]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        is_last = atomicAdd(scratch + bins, 1ull) == (unsigned long long)gridDim.x - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    const bool bad = __ldcg(scratch + bins + 1) != 0ull;
+    for (int i = threadIdx.x; i < bins; i += kThreads)
+        out[i] = bad ? nanf("")
+                     : fix_to_float((long long)__ldcg(scratch + i)) * kFixInv * inv_vol;
+}
+
+// d(profile)/dx: only the z components, (g[t][i1] - g[t][i0]) scale / vol
+__global__ void k_z_profile_vjp(const float* __restrict__ x, const int32_t* __restrict__ types,
+                                int64_t n, int T, int nb, float scale, float inv_vol,
+                                const float* __restrict__ g, float* __restrict__ gx) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const ZBin b = z_bin(x[3 * i + 2], scale, nb);
+        const int t = types[i];
+        float d = nanf("");
+        if (b.ok && t >= 0 && t < T)
+            d = (__ldg(g + t * nb + b.i1) - __ldg(g + t * nb + b.i0)) * inv_vol * scale;
+        gx[3 * i] = 0.0f;
+        gx[3 * i + 1] = 0.0f;
+        gx[3 * i + 2] = d;
+    }
+}
+
 // ------------------------------------------------------------ host glue ---
 int make_plan(hpf_ctx* c, cufftHandle* plan, cufftType type, int batch, size_t* ws) {
     int n[3] = {c->n0, c->n1, c->n2};
@@ -1133,6 +1245,16 @@ int hpf_ctx_set_functional(hpf_ctx* c, const double* Q, const double* b, double 
     return HPF_OK;
 }
 
+int hpf_ctx_set_functional_chi(hpf_ctx* c, const void* chi, int chi_f64, int with_chi,
+                               double kappa, double rho0, double a, double sigma, void* stream) {
+    if (!c || (with_chi && !chi) || !(kappa != 0.0) || !(rho0 != 0.0)) return HPF_ERR_ARG;
+    k_functional_chi<<<1, 256, 0, as_stream(stream)>>>(
+        c->d_fun, c->T, with_chi && !chi_f64 ? (const float*)chi : nullptr,
+        with_chi && chi_f64 ? (const double*)chi : nullptr, kappa, rho0, a, sigma);
+    HPF_LAUNCH_CHECK();
+    return HPF_OK;
+}
+
 int hpf_get_error(hpf_ctx* c, void* stream, int* code) {
     if (!c || !code) return HPF_ERR_ARG;
     int h = 0;
@@ -1208,6 +1330,34 @@ int hpf_kspace_sums(hpf_ctx* c, const void* phi_fourier, const void* psi_k,
         default: HPF_KSS(0); break;
     }
 #undef HPF_KSS
+    HPF_LAUNCH_CHECK();
+    return HPF_OK;
+}
+
+int hpf_z_profile(const float* x, const int32_t* types, int64_t n, int T, int n_bins, double Lz,
+                  double bin_volume, void* scratch, float* out, void* stream) {
+    if (n < 0 || T < 1 || n_bins < 1 || !(Lz > 0) || !(bin_volume > 0) || !scratch || !out ||
+        (n > 0 && (!x || !types)) || (int64_t)T * n_bins > (1 << 28))
+        return HPF_ERR_ARG;
+    const size_t smem = sizeof(unsigned long long) * (size_t)T * n_bins;
+    const int in_shared = smem <= 32 * 1024;
+    // four blocks per SM: each folds its own bins into the total
+    const int grid = (int)std::min<int64_t>(grid_for(n, kThreads), 2 * HPF_REDUCE_GRID);
+    k_z_profile<<<grid, kThreads, in_shared ? smem : 0, as_stream(stream)>>>(
+        x, types, n, T, n_bins, (float)(n_bins / Lz), (float)(1.0 / bin_volume),
+        (unsigned long long*)scratch, out, in_shared);
+    HPF_LAUNCH_CHECK();
+    return HPF_OK;
+}
+
+int hpf_z_profile_vjp(const float* x, const int32_t* types, int64_t n, int T, int n_bins,
+                      double Lz, double bin_volume, const float* g, float* gx, void* stream) {
+    if (n < 0 || T < 1 || n_bins < 1 || !(Lz > 0) || !(bin_volume > 0) ||
+        (n > 0 && (!x || !types || !g || !gx)))
+        return HPF_ERR_ARG;
+    if (n == 0) return HPF_OK;
+    k_z_profile_vjp<<<grid_for(n, kThreads), kThreads, 0, as_stream(stream)>>>(
+        x, types, n, T, n_bins, (float)(n_bins / Lz), (float)(1.0 / bin_volume), g, gx);
     HPF_LAUNCH_CHECK();
     return HPF_OK;
 }

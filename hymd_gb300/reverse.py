@@ -47,7 +47,7 @@ import torch
 from torch.utils.checkpoint import checkpoint
 
 from . import _lib
-from .adjoint import functional_coefficients
+from .adjoint import KINDS, functional_coefficients
 
 
 class ForceModel:
@@ -93,6 +93,17 @@ class ForceModel:
             self.group_masks = [md.group == g for g in range(self.thermo.n_groups)]
 
     def set_chi(self, chi):
+        if (chi.is_cuda and chi.get_device() == self.md.r.get_device() and chi.is_contiguous()
+                and tuple(chi.shape) == (self.T, self.T)
+                and chi.dtype in (torch.float32, torch.float64) and self.kind in KINDS):
+            # on the device, in stream order: no copy to the host per step
+            a = 0.0 if self.kind == "SquaredPhi" else self.a
+            _lib.call("hpf_ctx_set_functional_chi", self.pm._h, _lib.ptr(chi.detach()),
+                      int(chi.dtype == torch.float64), int(self.kind == "DefaultWithChi"),
+                      self.kappa, self.rho0, a, self.sigma, _lib.stream_ptr())
+            self.pm._functional = None
+            self._key = None
+            return
         Q, b, c = functional_coefficients(self.kind, chi.detach().cpu().numpy(), self.kappa,
                                           self.rho0, self.a)
         key = (Q.tobytes(), b.tobytes(), c, self.sigma)
@@ -305,9 +316,49 @@ def respa_step(x, v, f_field, f_bond, chi, model, step=None):
     return x, v, f_field, f_bond
 
 
+class _ZProfile(torch.autograd.Function):
+    """z_profile as one launch each way (hpf_z_profile)."""
+
+    @staticmethod
+    def forward(ctx, x, types, n_types, n_bins, box):
+        vol = box[0] * box[1] * box[2] / n_bins
+        scratch = torch.zeros(n_types * n_bins + 2, dtype=torch.int64, device=x.device)
+        out = torch.empty((n_types, n_bins), dtype=torch.float32, device=x.device)
+        _lib.call("hpf_z_profile", _lib.ptr(x), _lib.ptr(types), x.shape[0], n_types, n_bins,
+                  box[2], vol, _lib.ptr(scratch), _lib.ptr(out), _lib.stream_ptr())
+        ctx.save_for_backward(x, types)
+        ctx.args = (n_types, n_bins, box, vol)
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        x, types = ctx.saved_tensors
+        n_types, n_bins, box, vol = ctx.args
+        if torch.is_grad_enabled():
+            # create_graph: the derivative in operations torch can follow
+            with torch.enable_grad():
+                y = x.detach().requires_grad_(True)
+                p = _z_profile_torch(y, types, n_types, n_bins, box)
+            (gx,) = torch.autograd.grad(p, y, g, create_graph=True)
+            return gx, None, None, None, None
+        gx = torch.empty_like(x)
+        g = g.contiguous()
+        _lib.call("hpf_z_profile_vjp", _lib.ptr(x), _lib.ptr(types), x.shape[0], n_types, n_bins,
+                  box[2], vol, _lib.ptr(g), _lib.ptr(gx), _lib.stream_ptr())
+        return gx, None, None, None, None
+
+
 def z_profile(x, types, n_types, n_bins, box):
     """Per-type number density along z (beads / nm^3) with linear binning
     onto bin centres (periodic), differentiable in the positions."""
+    if (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and types.is_cuda
+            and types.dtype == torch.int32 and types.is_contiguous() and x.shape[0] > 0
+            and x.dim() == 2 and x.shape[1] == 3):
+        return _ZProfile.apply(x, types, n_types, n_bins, [float(b) for b in box])
+    return _z_profile_torch(x, types, n_types, n_bins, box)
+
+
+def _z_profile_torch(x, types, n_types, n_bins, box):
     Lz = box[2]
     s = x[:, 2] * (n_bins / Lz) - 0.5
     i0 = torch.floor(s).detach()

@@ -150,6 +150,12 @@ int hpf_ctx_get_spectral_tile(const hpf_ctx* ctx, int* width, int* allowed_mask)
  * width sigma (hymd/hamiltonian.py:74-486, H at :57-71).  Q is T*T row-major. */
 int hpf_ctx_set_functional(hpf_ctx* ctx, const double* Q, const double* b, double c,
                            double sigma);
+/* The same for the reference's functionals (hymd/hamiltonian.py:74-486) from
+ * their parameters, formed on the device in stream order: chi device
+ * float / double [T][T] (used symmetrised, its diagonal unused) with with_chi,
+ * else no chi term. */
+int hpf_ctx_set_functional_chi(hpf_ctx* ctx, const void* chi, int chi_f64, int with_chi,
+                               double kappa, double rho0, double a, double sigma, void* stream);
 /* First error recorded by a device-side check since the last call; clears
  * it.  Synchronises the stream. */
 int hpf_get_error(hpf_ctx* ctx, void* stream, int* code);
@@ -584,6 +590,14 @@ int hpf_respa_step_paint(hpf_respa_plan* plan, float* r, float* v, float* f_bond
                          const double* randoms, int* counter, double* state, int* d_err,
                          void* stream);
 
+/* Per-type number density along z, linear binning onto bin centres: out
+ * float[T][n_bins]; scratch: zeroed uint64[T n_bins + 2].  The sums do not
+ * depend on the order of the beads.  A non-finite position or a type out of
+ * range makes the profile NaN.  _vjp: gx float[n][3] from g = dL/d out. */
+int hpf_z_profile(const float* x, const int32_t* types, int64_t n, int T, int n_bins, double Lz,
+                  double bin_volume, void* scratch, float* out, void* stream);
+int hpf_z_profile_vjp(const float* x, const int32_t* types, int64_t n, int T, int n_bins,
+                      double Lz, double bin_volume, const float* g, float* gx, void* stream);
 /* Reverse mode of hpf_respa_step (without barostat): r, v, f_bonded and the
  * slow forces are the step's INPUTS; gx, gv, gf hold the cotangents of its
  * outputs r, v, f_bonded and are overwritten with the gradients of the inputs;
