@@ -63,12 +63,15 @@ def _set(pm, Q, b, c, sigma):
     pm._functional = None  # the cached key no longer describes the context
 
 
-def _energy(pm, pos, typ, masses, Q, b, c):
-    T = pm.n_types
-    out = torch.zeros(32, dtype=torch.float64, device=pm.device)
+def _queue_energy(pm, pos, typ, masses):
+    """The FP64 sums of W, queued; they end up in pm._report[:32]."""
     _lib.call("hpf_energy_fp64", pm._h, _lib.ptr(pos), _lib.ptr(typ), pos.shape[0],
-              _lib.dvec(masses), None, None, 0.0, _lib.ptr(out), _lib.stream_ptr())
-    o = out.cpu().numpy()
+              _lib.dvec(masses), None, None, 0.0, _lib.ptr(pm._report), _lib.stream_ptr())
+
+
+def _energy(pm, Q, b, c):
+    T = pm.n_types
+    o = pm._report[:32].cpu().numpy()
     V = float(np.prod(pm.BoxSize))
     means = o[16:16 + T]
     return V * (0.5 * means @ Q @ means + b @ means + c) + 0.5 * V * o[0]
@@ -78,9 +81,21 @@ class _FieldEnergy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, positions, chi, kappa, sigma, pm, types, masses, kind, rho0, a, ref_grad):
         k, s = float(kappa), float(sigma)
-        Q, b, c = functional_coefficients(kind, chi.detach().cpu().numpy(), k, rho0, a)
-        _set(pm, Q, b, c, s)
-        W = _energy(pm, positions, types, masses, Q, b, c)
+        if (chi.is_cuda and chi.get_device() == positions.get_device() and chi.is_contiguous()
+                and chi.dtype in (torch.float32, torch.float64) and kind in KINDS):
+            # the sums need the functional on the device only: queued with chi
+            # from there, while the host fetches chi for W's k = 0 part
+            _lib.call("hpf_ctx_set_functional_chi", pm._h, _lib.ptr(chi.detach()),
+                      int(chi.dtype == torch.float64), int(kind == "DefaultWithChi"), k, rho0,
+                      0.0 if kind == "SquaredPhi" else a, s, _lib.stream_ptr())
+            pm._functional = None
+            _queue_energy(pm, positions, types, masses)
+            Q, b, c = functional_coefficients(kind, chi.detach().cpu().numpy(), k, rho0, a)
+        else:
+            Q, b, c = functional_coefficients(kind, chi.detach().cpu().numpy(), k, rho0, a)
+            _set(pm, Q, b, c, s)
+            _queue_energy(pm, positions, types, masses)
+        W = _energy(pm, Q, b, c)
         ctx.pm, ctx.types, ctx.masses, ctx.kind = pm, types, masses, kind
         ctx.rho0, ctx.a, ctx.kappa, ctx.sigma = rho0, a, k, s
         ctx.Q, ctx.b, ctx.c = Q, b, c
@@ -98,7 +113,7 @@ class _FieldEnergy(torch.autograd.Function):
         need_p = any(ctx.needs_input_grad[1:4])
         grad_x = torch.empty_like(positions) if need_x else None
         P = T * (T + 1) // 2
-        sums = torch.zeros(P + 1 + T, dtype=torch.float64, device=positions.device) if need_p \
+        sums = torch.empty(P + 1 + T, dtype=torch.float64, device=positions.device) if need_p \
             else None
         if need_x and ctx.ref_grad:
             # minus the MD force (the readout of the spectral gradient)

@@ -55,7 +55,7 @@ __global__ void k_bonds(float* __restrict__ f, const float* __restrict__ r, int6
         acc[2] += (double)vir.y;
         acc[3] += (double)vir.z;
     }
-    grid_reduce_store<4>(acc, ws_partials(out), ws_ticket(out), out, false);
+    grid_reduce_store<4>(acc, ws_partials(out), ws_ticket(out), out, false, err);
 }
 
 __global__ void k_angles(float* __restrict__ f, const float* __restrict__ r, int64_t n,
@@ -84,7 +84,7 @@ __global__ void k_angles(float* __restrict__ f, const float* __restrict__ r, int
         acc[2] += (double)vir.y;
         acc[3] += (double)vir.z;
     }
-    grid_reduce_store<4>(acc, ws_partials(out), ws_ticket(out), out, false);
+    grid_reduce_store<4>(acc, ws_partials(out), ws_ticket(out), out, false, err);
 }
 
 __global__ void k_dihedrals(float* __restrict__ force, const float* __restrict__ r, int64_t n,
@@ -120,7 +120,7 @@ __global__ void k_dihedrals(float* __restrict__ force, const float* __restrict__
         for (int q = 0; q < 4; ++q) add3(force, idx[q], F[q]);
         acc[0] += (double)e;
     }
-    grid_reduce_store<1>(acc, ws_partials(out), ws_ticket(out), out, false);
+    grid_reduce_store<1>(acc, ws_partials(out), ws_ticket(out), out, false, err);
 }
 
 __global__ void k_dipole_redistribute(float* __restrict__ fob, int64_t n,

@@ -844,10 +844,12 @@ __device__ __forceinline__ bool grid_reduce_store_f(float (&vf)[K], double* part
     return false;
 }
 
+// err (may be NULL): a device error word, copied to out[7] once every block has
+// had its say, so that a caller reads results and error in one transfer.
 template <int K>
 __device__ __forceinline__ void grid_reduce_store(double (&v)[K], double* partials,
                                                   unsigned int* ticket, double* out,
-                                                  bool accumulate) {
+                                                  bool accumulate, const int* err = nullptr) {
     __shared__ double red[K * 32];
     __shared__ bool is_last;
     block_reduce<K>(v, red);
@@ -873,6 +875,7 @@ __device__ __forceinline__ void grid_reduce_store(double (&v)[K], double* partia
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < K; ++k) out[k] = (accumulate ? out[k] : 0.0) + acc[k];
+        if (K < 8 && err) out[7] = (double)*(const volatile int*)err;
         *ticket = 0u;
     }
 }

@@ -21,6 +21,7 @@ from . import _lib
 from .hamiltonian import quadratic_form
 
 _REGISTRY = {}
+_REGISTRY_FOURIER = {}
 
 
 class ParticleMesh:
@@ -47,7 +48,11 @@ class ParticleMesh:
         _lib.call("hpf_ctx_box_state", self._h, _lib.ctypes.byref(st))
         self.box_state_ptr = st.value
         self._functional = None
-        self.ws = _lib.new_workspace(self.device)
+        # energy sums, then the workspace of the kinetic energy: its result
+        # follows the sums, so that a print step reads both in one transfer
+        self._report = torch.zeros(32 + _lib.HPF_OUT_DOUBLES, dtype=torch.float64,
+                                   device=self.device)
+        self.ws = self._report[32:]
 
     # -- allocation helpers -------------------------------------------------
     def real_field(self, *lead):
@@ -172,26 +177,20 @@ class _DevicePtrArray:
 
 def _stack_base(lst, lead_shape, dtype, name):
     """Return the stacked tensor that the list elements are views of."""
-    flat = []
-
-    def walk(x):
-        if isinstance(x, (list, tuple)):
-            for y in x:
-                walk(y)
-        else:
-            flat.append(x)
-
-    walk(lst)
+    flat = [y for x in lst for y in (x if isinstance(x, (list, tuple)) else (x,))]
     first = flat[0]
     _lib.require_cuda(first, name + "[0]", dtype)
-    per = first.numel() * first.element_size()
-    for i, x in enumerate(flat):
-        if x.dtype != dtype or x.data_ptr() != first.data_ptr() + i * per or not x.is_contiguous():
+    p, per = first.data_ptr(), first.numel() * first.element_size()
+    for x in flat:
+        if x.dtype != dtype or x.data_ptr() != p or not x.is_contiguous():
             raise ValueError(f"{name} must be views of one stacked tensor as created by "
                              "initialize_pm")
-    base = torch.as_strided(first, (len(flat),) + tuple(first.shape),
-                            (first.numel(),) + tuple(first.stride()))
-    return base.reshape(tuple(lead_shape) + tuple(first.shape))
+        p += per
+    shape = tuple(lead_shape) + tuple(first.shape)
+    strides = [1] * len(shape)
+    for d in range(len(shape) - 1, 0, -1):
+        strides[d - 1] = strides[d] * shape[d]
+    return torch.as_strided(first, shape, strides)
 
 
 def initialize_pm(pmesh, config, comm=None):
@@ -246,6 +245,7 @@ def initialize_pm(pmesh, config, comm=None):
     field_list = [phi, phi_fourier, force_on_grid, v_ext_fourier, v_ext, phi_transfer,
                   phi_laplacian]
     _REGISTRY[phi_all.data_ptr()] = pm
+    _REGISTRY_FOURIER[phi_fourier_all.data_ptr()] = pm
     pm.fields = dict(phi=phi_all, phi_fourier=phi_fourier_all, force=force_all,
                      v_ext=v_ext_all, phi_laplacian=phi_lap_all)
     return pm, field_list, elec_common_list, coulomb_list
@@ -327,22 +327,30 @@ def _find_pm_for_force(force_all):
 
 
 def energy_fp64(pm, positions, types, masses, hamiltonian, charges=None, type_charges=None,
-                elec_factor=0.0):
+                elec_factor=0.0, velocity=None):
     """FP64 energy and pressure sums of the current positions (hpf_energy_fp64).
 
-    Returns dict(W, A, B[3], Eq, C0, C[3], means[T], V): W = V w(means) + V/2 A."""
+    Returns dict(W, A, B[3], Eq, C0, C[3], means[T], V): W = V w(means) + V/2 A;
+    with velocity also v2 = sum v^2."""
     T = pm.n_types
     Q, b, c, sigma = pm.set_functional(hamiltonian)
     pos = _lib.require_cuda(positions, "positions", torch.float32)
     n = pos.shape[0]
     typ = _types32(types, n)
     q = None if charges is None else _lib.require_cuda(charges, "charges", torch.float32, (n,))
-    out = torch.zeros(32, dtype=torch.float64, device=pm.device)
     qt = _lib.dvec(list(type_charges)) if type_charges is not None else None
+    vel = None if velocity is None else _lib.require_cuda(velocity, "velocity", torch.float32)
+    st = _lib.stream_ptr()
     _lib.call("hpf_energy_fp64", pm._h, _lib.ptr(pos), _lib.ptr(typ), n,
-              _lib.dvec(_masses(masses, T)), _lib.ptr(q), qt, float(elec_factor), _lib.ptr(out),
-              _lib.stream_ptr())
-    return decode_energy_sums(out.cpu().numpy(), Q, b, c, sigma, float(np.prod(pm.BoxSize)), T)
+              _lib.dvec(_masses(masses, T)), _lib.ptr(q), qt, float(elec_factor),
+              _lib.ptr(pm._report), st)
+    if vel is not None:
+        _lib.call("hpf_sum_v2", _lib.ptr(vel), vel.shape[0], _lib.ptr(pm.ws), st)
+    o = pm._report[:33].cpu().numpy()
+    e = decode_energy_sums(o, Q, b, c, sigma, float(np.prod(pm.BoxSize)), T)
+    if vel is not None:
+        e["v2"] = float(o[32])
+    return e
 
 
 def decode_energy_sums(o, Q, b, c, sigma, V, T):
@@ -374,10 +382,8 @@ def compute_field_and_kinetic_energy(phi, phi_q, psi, velocity, hamiltonian, pos
             raise ValueError("PIC_Spectral energy needs a preceding update_field_force_q")
         fac = config.coulomb_constant / config.dielectric_const
     e = energy_fp64(pm, positions, types, config.m, hamiltonian, charges=charges,
-                    elec_factor=fac)
-    vel = _lib.require_cuda(velocity, "velocity", torch.float32)
-    _lib.call("hpf_sum_v2", _lib.ptr(vel), vel.shape[0], _lib.ptr(pm.ws), _lib.stream_ptr())
-    ke = 0.5 * float(config.mass) * float(pm.ws[0])
+                    elec_factor=fac, velocity=velocity)
+    ke = 0.5 * float(config.mass) * e["v2"]
     wq = 0.0
     if charges is not None:
         wq = 0.5 * e["V"] * e["Eq"] - float(config.self_energy or 0.0)
@@ -455,7 +461,7 @@ def update_field_force_q_GPE(conv_fun, phi, types, charges, phi_q, phi_q_fourier
     qt = [float(x) for x in (config.type_charges or [0.0] * T)]
     ef = pm.gpe["elec_field"] if hasattr(pm, "gpe") else pm.real_field(3)
     vb = pm.gpe["vbar"] if hasattr(pm, "gpe") else pm.real_field(T)
-    dot = pm.real_field()
+    dot = torch.empty(pm.Nmesh, dtype=torch.float32, device=pm.device)
     pol = getattr(pm, "gpe_pol", None)
     if pol is None:
         pol = pm.gpe_pol = pm.real_field()
@@ -497,10 +503,9 @@ def comp_laplacian(phi_fourier, phi_transfer, phi_laplacian, hamiltonian, config
 
 
 def _pm_of_fourier(phi_fourier):
-    p = phi_fourier[0].data_ptr()
-    for pm in _REGISTRY.values():
-        if pm.fields["phi_fourier"].data_ptr() == p:
-            return pm
+    pm = _REGISTRY_FOURIER.get(phi_fourier[0].data_ptr())
+    if pm is not None:
+        return pm
     raise ValueError("phi_fourier was not created by hymd_gb300.field.initialize_pm")
 
 

@@ -419,7 +419,7 @@ _WS = {}
 
 
 def _ws(device, key):
-    k = (str(device), key)
+    k = (device, key)
     if k not in _WS:
         _WS[k] = _lib.new_workspace(device)
     return _WS[k]
@@ -447,18 +447,21 @@ def _dev_box(box, device):
 
 def _err(device):
     """Device int32 error word shared by the bonded entry points."""
-    k = (str(device), "err")
+    k = (device, "err")
     if k not in _WS:
         _WS[k] = torch.zeros(8, dtype=torch.int32, device=device)
     return _WS[k]
 
 
-def _check_err(device):
-    e = _err(device)
-    code = int(e[0].item())
+def _results(ws, err):
+    """Host copy of a call's results ws[:8]; the error word comes with them
+    (ws[7]), so that one transfer answers both."""
+    out = ws[:8].cpu().numpy()
+    code = int(out[7])
     if code:
-        e.zero_()
-        raise _lib.HPFError("bonded device check", int(code))
+        err.zero_()
+        raise _lib.HPFError("bonded device check", code)
+    return out
 
 
 # Every device argument below is bound to a local name until the library call
@@ -483,8 +486,7 @@ def compute_bond_forces(f, r, box, a, b, r0, k, sync=True):
               _lib.stream_ptr())
     if not sync:
         return ws
-    out = ws[:4].cpu().numpy()
-    _check_err(dev)
+    out = _results(ws, err)
     return float(out[0]), out[1:4].astype(np.float32)
 
 
@@ -502,8 +504,7 @@ def compute_angle_forces(f, r, box, a, b, c, t0, k, sync=True):
               _lib.ptr(err), _lib.stream_ptr())
     if not sync:
         return ws
-    out = ws[:4].cpu().numpy()
-    _check_err(dev)
+    out = _results(ws, err)
     return float(out[0]), out[1:4].astype(np.float32)
 
 
@@ -529,9 +530,7 @@ def compute_dihedral_forces(f, r, dipoles, transfer, box, a, b, c, d, coeff, dty
               _lib.ptr(ws), _lib.ptr(err), _lib.stream_ptr())
     if not sync:
         return ws
-    e = float(ws[0].item())
-    _check_err(dev)
-    return e
+    return float(_results(ws, err)[0])
 
 
 def dipole_forces_redistribution(f_on_bead, f_dipoles, trans_matrices, a, b, c, d, type_array,

@@ -17,7 +17,6 @@ cancel in single precision.  phi_laplacian is filled as in the reference
 import numpy as np
 import torch
 
-from . import _lib
 from .field import _pm_of, comp_laplacian, energy_fp64
 
 
@@ -36,12 +35,11 @@ def comp_pressure(phi, phi_q, psi, hamiltonian, velocities, config, phi_fourier,
         charges = getattr(pm, "pic_charges", None)
         fac = config.coulomb_constant / config.dielectric_const
         qt = list(config.type_charges)
-    e = energy_fp64(pm, positions, types, config.m, hamiltonian, charges=charges,
-                    type_charges=qt, elec_factor=fac)
+    # queued before the energies, whose result the host waits for
     comp_laplacian(phi_fourier, phi_transfer, phi_laplacian, hamiltonian, config)
-    vel = _lib.require_cuda(velocities, "velocities", torch.float32)
-    _lib.call("hpf_sum_v2", _lib.ptr(vel), vel.shape[0], _lib.ptr(pm.ws), _lib.stream_ptr())
-    ke = 0.5 * float(config.mass) * float(pm.ws[0])
+    e = energy_fp64(pm, positions, types, config.m, hamiltonian, charges=charges,
+                    type_charges=qt, elec_factor=fac, velocity=velocities)
+    ke = 0.5 * float(config.mass) * e["v2"]
     self_energy = float(config.self_energy or 0.0) if charges is not None else None
     return pressure_vector(e, ke, _host(bond_pr), _host(angle_pr), self_energy)
 

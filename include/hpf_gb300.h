@@ -413,7 +413,9 @@ int hpf_field_pic_step(hpf_ctx* ctx, float* pos, const int32_t* types, int64_t n
  * receives HPF_ERR_INDEX for out-of-range indices (the term is skipped).
  * box: DEVICE double[3] (e.g. the context box state), so that a captured
  * graph follows box changes made on the device. */
-/* cbf, hymd/compute_bond_forces.f90:1-61 */
+/* cbf, hymd/compute_bond_forces.f90:1-61
+ * out[7] of hpf_bonds / hpf_angles / hpf_dihedrals is the value of *d_err
+ * after the call (with d_err). */
 int hpf_bonds(float* f, const float* r, int64_t n, const double box[3], const int32_t* a,
               const int32_t* b, const float* r0, const float* k, int64_t nb, double* out,
               int* d_err, void* stream);
