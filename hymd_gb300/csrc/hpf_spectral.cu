@@ -50,6 +50,7 @@ struct SpecGeom {
     int n0, n1, n2, h, nzc;  // h = n2 / 2, nzc = h + 1
     int W, ws;               // columns per k-space tile, log2 W
     int ts;                  // stride of a grid's block in a k-space tile (float2)
+    int inplace;             // pass B: v's inverse transform in its own block
     int64_t M, Mc;
 };
 
@@ -255,7 +256,10 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     constexpr int NO = FIELDS ? 3 : 2;  // output columns per type
     float2* in = sm;                    // [T][Nx][W]
     float2* flt = sm + T * TS;          // FIELDS: filtered densities, [T][Nx][W]
-    float2* out = sm + (FIELDS ? 2 : 1) * T * TS;  // [NO T][Nx][W]
+    // FIELDS: [3T][Nx][W]; else [T][Nx][W], the x forces, then v's columns, or
+    // in place of v
+    float2* out = sm + (FIELDS ? 2 : 1) * T * TS;
+    float2* vout = g.inplace ? in : out + T * TS;
     for (int e = threadIdx.x; e < T * T; e += blockDim.x)
         sQ[(e / T) * kSpecMaxT + e % T] = fun->Q[e];
     for (int e = threadIdx.x; e < T; e += blockDim.x) sb[e] = fun->b[e];
@@ -270,7 +274,12 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     {
         constexpr int N1 = split1(N), N2 = N / N1;
         auto at_in = [&](int c, int e) -> float2& { return in[(c >> ws) * TS + e * W + (c & (W - 1))]; };
-        auto at_out = [&](int c, int e) -> float2& { return out[(c >> ws) * TS + e * W + (c & (W - 1))]; };
+        // column c of the inverse transforms: grid c >> ws of the output
+        auto at_out = [&](int c, int e) -> float2& {
+            const int gq = c >> ws, w = c & (W - 1);
+            if (FIELDS) return out[gq * TS + e * W + w];
+            return (gq & 1 ? vout : out)[(gq >> 1) * TS + e * W + w];
+        };
         // forward x transform of the densities
         auto ld = [&](int c, int n) {
             return __ldg(phi + (int64_t)(c >> ws) * g.Mc + n * plane + j0 + (c & (W - 1)));
@@ -350,14 +359,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
         // -i g_x v_to (the x force), e = 1 v_to itself (the y and z forces,
         // -i g_y v and -i g_z v, are formed from it in pass C: g_y and g_z
         // do not vary along x), e = 2 the filtered density
-        const int items = cout * N2;
-        for (int it = threadIdx.x; it < items; it += blockDim.x) {
-            const int n2 = N2 == 1 ? 0 : div_inv(it, cout, inv_cout);
-            const int c = it - n2 * cout;
-            const int gq = c >> ws, w = c & (W - 1);
-            const int to = gq / NO, e = gq - to * NO;
+        auto load1 = [&](int to, int w, int n2, int e, float2 (&a)[N1]) {
             const float2* vt = (FIELDS && e == 2 ? flt : in) + to * TS + w;
-            float2 a[N1];
 #pragma unroll
             for (int i = 0; i < N1; ++i) {
                 const int ix = N2 * i + n2;
@@ -365,6 +368,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                 const float gx = ix == N / 2 ? 0.0f : (ix <= N / 2 ? ix : ix - N) * kf0;
                 a[i] = e ? v : make_float2(gx * v.y, -gx * v.x);
             }
+        };
+        auto transform1 = [&](int n2, float2 (&a)[N1]) {
             reg_fft<N1, true>(a);
             if (N2 > 1) {
 #pragma unroll
@@ -373,8 +378,46 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                     a[k1] = c_mul(a[k1], make_float2(tw1.x, -tw1.y));
                 }
             }
+        };
+        const bool inplace = !FIELDS && g.inplace;
+        const int first = inplace ? cin : cout;
+        const float inv_first = inplace ? inv_cin : inv_cout;
+        const int items = first * N2;
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int n2 = N2 == 1 ? 0 : div_inv(it, first, inv_first);
+            const int c = it - n2 * first;
+            const int gq = c >> ws, w = c & (W - 1);
+            const int to = FIELDS ? gq / 3 : (inplace ? gq : gq >> 1);
+            const int e = FIELDS ? gq - 3 * to : (inplace ? 0 : gq & 1);
+            float2 a[N1];
+            load1(to, w, n2, e, a);
+            transform1(n2, a);
+            float2* dst = FIELDS ? out + gq * TS : (e ? vout : out) + to * TS;
 #pragma unroll
-            for (int k1 = 0; k1 < N1; ++k1) at_out(c, N2 * k1 + n2) = a[k1];
+            for (int k1 = 0; k1 < N1; ++k1) dst[(N2 * k1 + n2) * W + w] = a[k1];
+        }
+        if (inplace) {
+            // v in place: an item overwrites positions that other items of
+            // its column read, so whole columns go together, with a barrier
+            // between their loads and their stores
+            constexpr int CPR = kSpecThreads / N2;  // columns per round
+            const int n2 = threadIdx.x / CPR;
+            __syncthreads();
+            for (int c0 = 0; c0 < cin; c0 += CPR) {
+                const int c = c0 + threadIdx.x - n2 * CPR;
+                const bool on = n2 < N2 && c < cin;
+                const int to = c >> ws, w = c & (W - 1);
+                float2 a[N1];
+                if (on) {
+                    load1(to, w, n2, 1, a);
+                    transform1(n2, a);
+                }
+                __syncthreads();
+                if (on) {
+#pragma unroll
+                    for (int k1 = 0; k1 < N1; ++k1) in[to * TS + (N2 * k1 + n2) * W + w] = a[k1];
+                }
+            }
         }
         __syncthreads();
         // inverse x transforms, step 2: the force spectra
@@ -652,6 +695,7 @@ SpecGeom spec_geom(const hpf_ctx* c, int W) {
     g.W = W;
     g.ws = ilog2_host(g.W > 0 ? g.W : 1);
     g.ts = c->n0 * g.W + tile_pad(g.W);
+    g.inplace = 0;
     g.M = c->M;
     g.Mc = c->Mc;
     return g;
@@ -682,10 +726,10 @@ int with_planes(int n1, int h, F f) {
 #undef HPF_PLANE
     return HPF_ERR_ARG;
 }
-// a k-space tile: T density blocks in + 2T out, or (pic) 1 charge block in
-// + 2 out
-size_t tile_smem(const hpf_ctx* c, int W, bool pic = false) {
-    const int blocks = pic ? 3 : 3 * c->T;
+// a k-space tile: T density blocks in + 2T out (or 2T in all, in place), or
+// (pic) 1 charge block in + 2 out
+size_t tile_smem(const hpf_ctx* c, int W, bool pic = false, bool inplace = false) {
+    const int blocks = pic ? 3 : (inplace ? 2 : 3) * c->T;
     return sizeof(float2) * (size_t)blocks * (c->n0 * W + tile_pad(W));
 }
 
@@ -693,6 +737,13 @@ size_t tile_smem(const hpf_ctx* c, int W, bool pic = false) {
 size_t fields_smem(const hpf_ctx* c, int W) {
     return sizeof(float2) * (size_t)(5 * c->T) * (c->n0 * W + tile_pad(W));
 }
+
+// Whether a density tile of W columns transforms v in place: only where the
+// tile does not fit otherwise.  It costs one more barrier per round of columns
+// (10k melt 38.3 -> 38.9 us a step with every tile in place), and buys 128^3
+// meshes of three types the 16-column tile, whose every transform step has an
+// item for each thread (500k peptides 276 -> 268 us a step).
+bool tile_inplace(const hpf_ctx* c, int W) { return tile_smem(c, W) > kSpecTileSmem; }
 
 // The widest tile of W in {16, 8, 4} columns that divides n1, fits the
 // shared-memory budget and leaves a tile for every SM (4 when none does).
@@ -722,7 +773,7 @@ bool spectral_eligible(const hpf_ctx* c) {
 // + 1) columns split into whole tiles), within the shared-memory budget.
 bool spectral_tile_ok(const hpf_ctx* c, int W) {
     if (W != 4 && W != 8 && W != 16) return false;
-    return c->n1 % W == 0 && tile_smem(c, W) <= kSpecTileSmem;
+    return c->n1 % W == 0 && tile_smem(c, W, false, tile_inplace(c, W)) <= kSpecTileSmem;
 }
 
 // Select the k-space tile width (the autotuner's knob); the partials were
@@ -798,10 +849,11 @@ size_t spectral_ws_words(const hpf_ctx* c) { return 4 * (size_t)c->spec_max_tile
 // k_kspace_force's (out[0..3]) when non-null.
 int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st,
                          cudaEvent_t join) {
-    const SpecGeom g = spec_geom(c, c->spec_W);
+    SpecGeom g = spec_geom(c, c->spec_W);
+    g.inplace = tile_inplace(c, g.W);
     SpecScale sc;
     for (int t = 0; t < c->T; ++t) sc.s[t] = type_scale[t];
-    const int ps = (int)plane_smem(c), ts = (int)tile_smem(c, g.W);
+    const int ps = (int)plane_smem(c), ts = (int)tile_smem(c, g.W, false, g.inplace);
     if (with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto) {
             return launch_pdl(kf, dim3(c->n0, c->T), kSpecThreads, ps, st, c->d_acc,
                               c->d_spec_phi, g, sc, c->d_box, c->d_tw, nullptr) == cudaSuccess
