@@ -146,8 +146,12 @@ class RespaMD:
             raise _lib.HPFError("hpf_respa_plan_create", code)
         return h
 
-    # group sizes tried by the autotuner (beads per molecule group)
-    BLOCK_CANDIDATES = (12, 16, 24, 32, 36, 48, 64)
+    # group sizes tried by the autotuner (beads per molecule group): one warp
+    # per group up to 64, one CTA beyond.  Chains of four-body terms too short
+    # to need a CTA still run faster on one while there are few of them (5 of
+    # 40 beads among 6000: 88 -> 70 us a step on CTAs of one chain, 77 on CTAs
+    # of three; 133 of 60 beads among 200k: 201 -> 184 us).
+    BLOCK_CANDIDATES = (12, 16, 24, 32, 48, 64, 65, 128)
 
     def _tune_plan(self, packed, reps=4):
         """Molecule-group size of the fused inner kernel picked by timing it on
@@ -167,7 +171,8 @@ class RespaMD:
             a, b, m = _lib.I(), _lib.I(), _lib.I()
             _lib.call("hpf_respa_plan_info", plan, _lib.ctypes.byref(a), _lib.ctypes.byref(b),
                       _lib.ctypes.byref(m))
-            key = (a.value, m.value)
+            # one CTA per group beyond 64 beads: the same grouping may run either way
+            key = (a.value, m.value, c > 64 or m.value > 64)
             if key in seen:
                 _lib.lib().hpf_respa_plan_destroy(plan)
                 continue
