@@ -151,6 +151,12 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
 int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi, double* sums,
                  cudaStream_t st, const float* real_in = nullptr, bool filter = true,
                  const PicOut& o = PicOut{nullptr, nullptr, nullptr});
+// Maps of the charge chain's pass B on the density rho: 4 pi f H / k^2 and 4
+// pi f / k^2 (k^2 = 1 at k = 0), f H, f.  Grid layouts of pass C (k_spec_inv).
+enum SpecOp { kPoissonH = 0, kPoisson = 1, kFilter = 2, kIdentity = 3 };
+enum SpecOut { kDensity = 0, kPic = 1, kFields = 2 };
+int spectral_map(hpf_ctx* c, const SpecBufs& b, const float* real_in, int grids, int op, float fac,
+                 int mode, int first, int count, float* grid, float* aux, cudaStream_t st);
 // painted accumulators -> the grids and spectra of update_field
 bool spectral_fields_ok(const hpf_ctx* c);
 int spectral_fields(hpf_ctx* c, const float* type_scale, float* phi, float2* phi_k, float* force,

@@ -442,13 +442,14 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
 // k_kspace_pic): one charge-density column set in, psi = 4 pi f H rho / k^2
 // (k^2 = 1 at k = 0) out as -i k'_x psi (grid 0) and psi (grid 1), pass C
 // forming psi and the field components -i k'_d psi from them; sum of
-// w_k rho(k).psi(k) over the half spectrum into sums[0].
+// w_k rho(k).psi(k) over the half spectrum into sums[0].  op selects the map
+// (SpecOp); blockIdx.y: the input grid.
 template <int N>
 __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_kspace_pic(const float2* __restrict__ rho, float2* __restrict__ out_spec, SpecGeom g,
                       const BoxState* __restrict__ bs, const Functional* __restrict__ fun,
                       float four_pi_fac, const float2* __restrict__ tw,
-                      double* sums, double* partials, unsigned int* ticket, int filter,
+                      double* sums, double* partials, unsigned int* ticket, int op,
                       float2* __restrict__ psi_k) {
     pdl_wait();
     extern __shared__ __align__(16) float2 sm[];
@@ -456,6 +457,8 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     const int W = g.W, ws = g.ws, TS = g.ts;
     const int64_t plane = (int64_t)g.n1 * g.nzc;
     const int j0 = blockIdx.x * W;
+    rho += (int64_t)blockIdx.y * g.Mc;
+    out_spec += 2 * (int64_t)blockIdx.y * g.Mc;
     float2* in = sm;        // [Nx][W]
     float2* out = sm + TS;  // [2][Nx][W]: -i g_x psi, psi
     tile_columns(col, g, j0, bs);
@@ -491,11 +494,12 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                 const int ix = N2 * i + n2;
                 const float kx = (ix <= N / 2 ? ix : ix - N) * kf0;
                 float k2 = kx * kx + ci.ky * ci.ky + ci.kz * ci.kz;
-                const float Hk = filter ? expf(-s2h * k2) : 1.0f;
+                const float Hk =
+                    op == kPoissonH || op == kFilter ? expf(-s2h * k2) : 1.0f;
                 if (ix == 0 && ci.origin) k2 = 1.0f;  // k.normp(p=2, zeromode=1)
                 const float2 r = in[fx::pos(ix) * W + w];
                 const float2 rq = make_float2(r.x * invM, r.y * invM);
-                const float sc = four_pi_fac * Hk / k2;
+                const float sc = op <= kPoisson ? four_pi_fac * Hk / k2 : four_pi_fac * Hk;
                 const float2 v = make_float2(rq.x * sc, rq.y * sc);
                 if (psi_k && e) psi_k[ix * plane + j0 + w] = v;
                 if (sums && e == 0)
@@ -546,12 +550,11 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
 // Output grid gi comes from pass B's grid src: -i g_x v (x force) as is, v
 // times -i g_y (a function of the row ky) or -i g_z (of the column kz) for the
 // y and z forces, v (psi, the external potential) and the filtered density as
-// they are.
+// they are (SpecOut):
 //   kDensity: gi = 3 t + d, force grids of `grid`
 //   kPic:     gi = 0 psi (`aux`), 1..3 E_d (`grid`)
 //   kFields:  gi < 3 T as kDensity, then T filtered densities (`aux`), then T
 //             external potentials (`aux2`)
-enum SpecOut { kDensity = 0, kPic = 1, kFields = 2 };
 template <int NY, int HZ>
 __global__ void __launch_bounds__(kSpecThreads, 2)
     k_spec_inv(const float2* __restrict__ spec, float* __restrict__ grid, SpecGeom g,
@@ -948,7 +951,7 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
     int r = with_kspace(c->n0, [&](auto, auto kp, auto) {
         return launch_pdl(kp, c->spec_tiles_pic, kSpecThreads, ts, st, b.spec_phi, b.spec, g,
                           c->d_box, c->d_fun, four_pi_fac, c->d_tw, sums, part, tick,
-                          filter ? 1 : 0, o.psi_k) == cudaSuccess
+                          (int)(filter ? kPoissonH : kPoisson), o.psi_k) == cudaSuccess
                    ? HPF_OK
                    : HPF_ERR_CUDA;
     });
@@ -964,4 +967,41 @@ int spectral_pic(hpf_ctx* c, const SpecBufs& b, float four_pi_fac, bool want_psi
         }) != HPF_OK)
         return HPF_ERR_CUDA;
     return HPF_OK;
+}
+
+// Linear maps of real grids on the charge chain's passes: `grids` of them
+// (real_in float[grids][M], or the charge accumulator when NULL) -> passes A
+// and B with the map op (scaled by fac) -> pass C's grids [first, first +
+// count) of the layout `mode` into grid / aux.  b's spectra hold grids and 2
+// grids half spectra.
+int spectral_map(hpf_ctx* c, const SpecBufs& b, const float* real_in, int grids, int op, float fac,
+                 int mode, int first, int count, float* grid, float* aux, cudaStream_t st) {
+    const SpecGeom g = spec_geom(c, c->spec_W_pic);
+    SpecScale sc;
+    for (int t = 0; t < grids; ++t) sc.s[t] = 1.0f;
+    const int ps = (int)plane_smem(c), ts = (int)tile_smem(c, g.W, true);
+    int r = with_planes(c->n1, c->n2 / 2, [&](auto kf, auto, auto kr) {
+        const cudaError_t e =
+            real_in ? launch_pdl(kr, dim3(c->n0, grids), kSpecThreads, ps, st, nullptr, b.spec_phi,
+                                 g, sc, c->d_box, c->d_tw, real_in)
+                    : launch_pdl(kf, dim3(c->n0, 1), kSpecThreads, ps, st,
+                                 c->d_acc + (int64_t)c->T * c->M, b.spec_phi, g, sc, c->d_box,
+                                 c->d_tw, nullptr);
+        return e == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
+    });
+    if (r != HPF_OK) return r;
+    r = with_kspace(c->n0, [&](auto, auto kp, auto) {
+        return launch_pdl(kp, dim3(c->spec_tiles_pic, grids), kSpecThreads, ts, st, b.spec_phi,
+                          b.spec, g, c->d_box, c->d_fun, fac, c->d_tw, nullptr, nullptr, nullptr,
+                          op, nullptr) == cudaSuccess
+                   ? HPF_OK
+                   : HPF_ERR_CUDA;
+    });
+    if (r != HPF_OK) return r;
+    return with_planes(c->n1, c->n2 / 2, [&](auto, auto ki, auto) {
+        return launch_pdl(ki, dim3(c->n0, count), kSpecThreads, ps, st, b.spec, grid, g, c->d_box,
+                          c->d_tw, first, mode, c->T, aux, nullptr) == cudaSuccess
+                   ? HPF_OK
+                   : HPF_ERR_CUDA;
+    });
 }
