@@ -991,6 +991,19 @@ int launch_readout(hpf_ctx* c, const float* fm, const float* pos, const int32_t*
     return e == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
 }
 
+int exec_r2c(hpf_ctx* c, const float* in, float2* out, int batch, cudaStream_t st);
+int exec_c2r(hpf_ctx* c, const float2* in, float* out, int batch, cudaStream_t st);
+
+// densities in d_grid -> force mesh in d_grid by the library FFTs
+int library_field_force(hpf_ctx* c, double* sums, cudaStream_t st) {
+    int r;
+    if ((r = exec_r2c(c, c->d_grid, c->d_spec_phi, c->T, st)) != HPF_OK) return r;
+    if ((r = launch_kspace_force(c, c->d_spec_phi, c->d_spec, nullptr, nullptr, sums, st)) !=
+        HPF_OK)
+        return r;
+    return exec_c2r(c, c->d_spec, c->d_grid, 3 * c->T, st);
+}
+
 SpecBufs main_bufs(hpf_ctx* c) { return SpecBufs{c->d_spec_phi, c->d_spec, c->d_grid, c->d_spec_ws}; }
 SpecBufs pic_bufs(hpf_ctx* c) {
     return SpecBufs{c->pic_spec_phi, c->pic_spec, c->pic_grid, c->pic_spec_ws};
@@ -1476,11 +1489,7 @@ int hpf_field_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
     }
     if ((r = do_paint(c, pos, types, nullptr, n, c->T, sc, c->d_grid, st, pos_scale)) != HPF_OK)
         return r;
-    if ((r = exec_r2c(c, c->d_grid, c->d_spec_phi, c->T, st)) != HPF_OK) return r;
-    if ((r = launch_kspace_force(c, c->d_spec_phi, c->d_spec, nullptr, nullptr, sums, st)) !=
-        HPF_OK)
-        return r;
-    if ((r = exec_c2r(c, c->d_spec, c->d_grid, 3 * c->T, st)) != HPF_OK) return r;
+    if ((r = library_field_force(c, sums, st)) != HPF_OK) return r;
     if (n > 0) return launch_readout(c, c->d_grid, pos, types, nullptr, n, c->T, force, kick, st);
     return HPF_OK;
 }
@@ -1646,15 +1655,27 @@ int hpf_field_pic_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
     // pass; at once where the deposits are still to be made or both chains run
     cudaEvent_t join = c->pending;
     c->pending = nullptr;
-    if (join && (!painted || charges)) {
+    if (join && (!painted || charges || !c->spec_fused)) {
         HPF_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
         join = nullptr;
     }
     int r;
     if (!c->spec_fused) {
         // the library-FFT path shares its plans' work area: one chain after
-        // the other; deposits made elsewhere are not taken
-        if (painted) return HPF_ERR_ARG;
+        // the other.  Density deposits made elsewhere are finalised here;
+        // with charges they are not taken (measured to gain nothing), nor
+        // with a barostat's scale (positions scaled by the readout)
+        if (painted && (pos_scale || charges)) return HPF_ERR_ARG;
+        if (painted) {
+            TypeScale sc;
+            for (int t = 0; t < c->T; ++t) sc.s[t] = (float)type_mass[t];
+            if ((r = do_paint(c, pos, types, nullptr, 0, c->T, sc, c->d_grid, st)) != HPF_OK ||
+                (r = library_field_force(c, sums, st)) != HPF_OK)
+                return r;
+            if (n > 0)
+                return launch_readout(c, c->d_grid, pos, types, nullptr, n, c->T, force, kick, st);
+            return HPF_OK;
+        }
         if ((r = hpf_field_step(c, pos, types, n, type_mass, force, sums, pos_scale,
                                 charges ? nullptr : kick, stream)) != HPF_OK)
             return r;

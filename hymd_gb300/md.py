@@ -689,8 +689,14 @@ class RespaMD:
 
     @property
     def _paint_fused(self):
-        return (self.FUSE_PAINT and self.plan is not None and self.pm.spectral == "fused"
+        # library-FFT meshes: without charges or a barostat (us a step,
+        # separate / fused paint: 3k melt 52.2 / 50.5, 50k melt 63.9 / 62.2,
+        # 300k membrane 321.6 / 316.6; with charges 8k 95.6 / 96.9, 100k 197.6
+        # / 195.1)
+        return (self.FUSE_PAINT and self.plan is not None
                 and (self.baro_args is None or self.baro_mode == 0)
+                and (self.pm.spectral == "fused"
+                     or (self.charges is None and self.baro_args is None))
                 and (self.charges is None or self.CONCURRENT_PIC))
 
     def _field(self, st, sums=None, pos_scale=None, kick=None, painted=False):
@@ -780,7 +786,7 @@ class RespaMD:
         128, 12k 97 / 96), so there the sums stay in line; so they do in a
         subclass with a second half of its own."""
         return (self._paint_fused and self.charges is None and self.baro_args is None
-                and type(self)._outer_rest is RespaMD._outer_rest)
+                and self.pm.spectral == "fused" and type(self)._outer_rest is RespaMD._outer_rest)
 
     def _inner_fused(self, st, defer=False):
         """First outer kick + all inner steps (+ the barostat's box update in

@@ -395,8 +395,8 @@ int hpf_pic_step_list(hpf_ctx* ctx, const float* pos, const float* charges, cons
  * update, which gives the same grid coordinates), and the density readout
  * scales the positions by (float)pos_scale[0] as it reads them and writes
  * them back (as hpf_scr_scale_positions would, without its launch).  On the
- * fused spectral path only (painted or the second stream); otherwise the
- * two calls run one after the other.
+ * library-FFT path the two calls run one after the other, and painted is
+ * taken without charges and pos_scale only (HPF_ERR_ARG).
  * The first call with charges allocates the charge chain's scratch (about
  * 3 Mc complex and 4 M real values) and must not be under stream capture
  * (HPF_ERR_ARG). */
