@@ -414,14 +414,16 @@ __global__ void k_kspace_pic(const float2* __restrict__ rho_raw, float2* __restr
 // accumulators are converted to double grids, transformed with a D2Z cuFFT
 // and reduced over the half spectrum in FP64.  Used where the reference
 // reports energies (print steps, barostat), never inside the MD step.
+// blockIdx.y: the grid.
 __global__ void k_paint_finalize_f64(unsigned long long* __restrict__ acc,
-                                     double* __restrict__ out, int64_t M, int G, TypeScaleD sc,
+                                     double* __restrict__ out, int64_t M, TypeScaleD sc,
                                      const BoxState* __restrict__ bs) {
-    const double inv_dV = 1.0 / bs->dV;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)G * M;
+    const double s = sc.s[blockIdx.y] * (1.0 / bs->dV) * (double)kFixInv;
+    acc += (int64_t)blockIdx.y * M;
+    out += (int64_t)blockIdx.y * M;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < M;
          e += (int64_t)gridDim.x * blockDim.x) {
-        const int g = (int)(e / M);
-        out[e] = (double)(long long)acc[e] * (sc.s[g] * inv_dV * (double)kFixInv);
+        out[e] = (double)(long long)acc[e] * s;
         acc[e] = 0ull;
     }
 }
@@ -815,10 +817,10 @@ int ensure_spec64(hpf_ctx* c) {
     return HPF_OK;
 }
 
-// The FP64 buffers and the D2Z plan (batch T+1: densities + charges) are
-// only needed for energies and gradients: created on first use.
-int ensure_d2z(hpf_ctx* c) {
-    if (c->has_d2z) return HPF_OK;
+// The FP64 buffers and the D2Z plans (T densities, T + 1 with the charges)
+// are only needed for energies and gradients: created on first use.
+int ensure_d2z(hpf_ctx* c, int q) {
+    if (c->has_d2z[q]) return HPF_OK;
     const int T = c->T;
     if (!c->d_grid64)
         HPF_CUDA_TRY(cudaMalloc(&c->d_grid64, sizeof(double) * (size_t)(T + 1) * c->M));
@@ -826,13 +828,13 @@ int ensure_d2z(hpf_ctx* c) {
     if (r != HPF_OK) return r;
     long long nn[3] = {c->n0, c->n1, c->n2};
     size_t ws = 0;
-    if (cufftCreate(&c->plan_d2z) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
-    if (cufftMakePlanMany64(c->plan_d2z, 3, nn, NULL, 1, c->M, NULL, 1, c->Mc, CUFFT_D2Z, T + 1,
+    if (cufftCreate(&c->plan_d2z[q]) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
+    if (cufftMakePlanMany64(c->plan_d2z[q], 3, nn, NULL, 1, c->M, NULL, 1, c->Mc, CUFFT_D2Z, T + q,
                             &ws) != CUFFT_SUCCESS) {
-        cufftDestroy(c->plan_d2z);
+        cufftDestroy(c->plan_d2z[q]);
         return HPF_ERR_CUFFT;
     }
-    c->has_d2z = true;
+    c->has_d2z[q] = true;
     return HPF_OK;
 }
 
@@ -853,21 +855,22 @@ int paint_f64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n, con
 }
 
 // Densities (fixed-point paint) as FP64 grids and their D2Z spectra in
-// d_spec64 (slots 0..T-1; slot T holds the charges when given, else zeros).
+// d_spec64 (slots 0..T-1; slot T holds the charges when given).
 int density_spectra_f64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n,
                         const double* type_mass, const float* charges, cudaStream_t st) {
-    int r = ensure_d2z(c);
+    const int q = charges ? 1 : 0;
+    int r = ensure_d2z(c, q);
     if (r != HPF_OK) return r;
     const int T = c->T;
     TypeScaleD sc;
     for (int t = 0; t < T; ++t) sc.s[t] = type_mass[t];
     sc.s[T] = 1.0;
     if ((r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK) return r;
-    k_paint_finalize_f64<<<grid_for((int64_t)(T + 1) * c->M, kThreads), kThreads, 0, st>>>(
-        c->d_acc, c->d_grid64, c->M, T + 1, sc, c->d_box);
+    k_paint_finalize_f64<<<dim3(grid_for(c->M, kThreads), T + q), kThreads, 0, st>>>(
+        c->d_acc, c->d_grid64, c->M, sc, c->d_box);
     HPF_LAUNCH_CHECK();
-    if (cufftSetStream(c->plan_d2z, st) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
-    if (cufftExecD2Z(c->plan_d2z, c->d_grid64, reinterpret_cast<cufftDoubleComplex*>(c->d_spec64)) !=
+    if (cufftSetStream(c->plan_d2z[q], st) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
+    if (cufftExecD2Z(c->plan_d2z[q], c->d_grid64, reinterpret_cast<cufftDoubleComplex*>(c->d_spec64)) !=
         CUFFT_SUCCESS)
         return HPF_ERR_CUFFT;
     return HPF_OK;
@@ -1085,7 +1088,8 @@ int hpf_ctx_destroy(hpf_ctx* c) {
     cudaFree(c->d_spec_phi);
     cudaFree(c->d_ws);
     cudaFree(c->d_err);
-    if (c->has_d2z) cufftDestroy(c->plan_d2z);
+    for (int q = 0; q < 2; ++q)
+        if (c->has_d2z[q]) cufftDestroy(c->plan_d2z[q]);
     cudaFree(c->d_grid64);
     cudaFree(c->d_spec64);
     cudaFree(c->gpe_grid);

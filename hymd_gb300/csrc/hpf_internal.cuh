@@ -55,8 +55,8 @@ struct hpf_ctx {
     void* fft_work;
     size_t fft_work_size;
     // FP64 energy path (created on first use, outside graph capture)
-    cufftHandle plan_d2z;     // batch T+1: T densities + charges
-    bool has_d2z;
+    cufftHandle plan_d2z[2];  // batch T densities; T + 1 with the charges
+    bool has_d2z[2];
     double* d_grid64;         // double[T+1][M]
     double2* d_spec64;        // double2[T+1][Mc]
     cufftHandle plan_r2c[HPF_MAX_TYPES + 1];   // batch b at index b (created lazily)
