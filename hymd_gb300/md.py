@@ -164,13 +164,24 @@ class RespaMD:
         arr = (_lib.P * 1)(_lib.ptr(slow))
         st = _lib.stream_ptr()
         best, seen, timings = None, set(), {}
+        largest, caps = 0, set()
+        four_body = len(packed[9]) > 0
         for c in self.BLOCK_CANDIDATES:
+            # a cap below the largest molecule gives that molecule's grouping
+            # again; without four-body terms a CTA lost to the warps on every
+            # melt and membrane timed, so it is not built where a warp will do
+            if max(c, largest) in caps or (c > 64 >= largest and not four_body):
+                continue
+            caps.add(max(c, largest))
             plan = self._make_plan(packed, c)
             if plan is None:
                 continue
             a, b, m = _lib.I(), _lib.I(), _lib.I()
             _lib.call("hpf_respa_plan_info", plan, _lib.ctypes.byref(a), _lib.ctypes.byref(b),
                       _lib.ctypes.byref(m))
+            if m.value > c:
+                largest = m.value
+                caps.add(largest)
             # one CTA per group beyond 64 beads: the same grouping may run either way
             key = (a.value, m.value, c > 64 or m.value > 64)
             if key in seen:
