@@ -24,6 +24,16 @@ __device__ __forceinline__ V3 load3(const float* r, int i) {
     return v3(r[3 * i], r[3 * i + 1], r[3 * i + 2]);
 }
 
+// Threads per block of k_dihedrals.  What bounds it is the latency of one
+// term: 30 uncoalesced coefficient loads, 15 sincos, the four-body force.  Up
+// to one full block per SM, small blocks spread the terms over SMs and L1s
+// that would otherwise have none (9400 terms fill 37 of the SMs in full
+// blocks): 25 -> 14.5 us for them, and the bonded forces of those 500k-bead
+// peptides 217 -> 200 us.  Beyond that every SM has work, and the extra partial
+// sums buy nothing.  Bonds and angles, a few loads a term, measured the same
+// either way (9.5 us for 19800 and 9600) and stay with full blocks.
+inline int dih_threads(int64_t n) { return n <= (int64_t)152 * kThreads ? 64 : kThreads; }
+
 __device__ __forceinline__ void add3(float* f, int i, V3 v) {
     atomicAdd(f + 3 * i, v.x);
     atomicAdd(f + 3 * i + 1, v.y);
@@ -157,8 +167,8 @@ __global__ void k_dipole_redistribute(float* __restrict__ fob, int64_t n,
     }
 }
 
-int grid_for(int64_t work) {
-    int64_t g = (work + kThreads - 1) / kThreads;
+int grid_for(int64_t work, int threads = kThreads) {
+    int64_t g = (work + threads - 1) / threads;
     if (g < 1) g = 1;
     if (g > HPF_REDUCE_BLOCKS) g = HPF_REDUCE_BLOCKS;
     return (int)g;
@@ -293,9 +303,10 @@ int hpf_dihedrals(float* f, const float* r, int64_t n, float* dipoles, float* tr
         return HPF_ERR_ARG;
     cudaStream_t st = as_stream(stream);
     HPF_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(float) * 3 * n, st));
-    k_dihedrals<<<grid_for(nd), kThreads, 0, st>>>(f, r, n, dipoles, transfer, box, a, b, c, d,
-                                                   coeff, dtype, last, nd, dipole_flag, out,
-                                                   d_err);
+    const int threads = dih_threads(nd);
+    k_dihedrals<<<grid_for(nd, threads), threads, 0, st>>>(f, r, n, dipoles, transfer, box, a, b,
+                                                           c, d, coeff, dtype, last, nd,
+                                                           dipole_flag, out, d_err);
     HPF_LAUNCH_CHECK();
     return HPF_OK;
 }
