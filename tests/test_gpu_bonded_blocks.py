@@ -1,11 +1,10 @@
 """The per-term bonded kernels over their launch shapes (four-body terms: small
-blocks up to
-one full block per SM, full ones beyond; all: a thread handling several
-terms once the grid is full) against the FP64 C restatement.  Zigzag
-segments away from the walls: a difference of two neighbouring positions is
-exact, a bond's stretch of 0.05 carries 3e-8 / 0.05 = 6e-7 of rounding and the
-cosine series and angles the same order, so forces agree to 1e-5 rel-RMS and
-energies (sums of like-signed terms) to 1e-6."""
+blocks up to one full block per SM, full ones beyond; all: several terms a
+thread once the grid is full) against the FP64 C restatement.  Zigzag segments
+away from the walls: a difference of two neighbouring positions is exact, a
+bond's stretch of 0.05 carries 3e-8 / 0.05 = 6e-7 of rounding and the cosine
+series and angles the same order, so forces agree to 1e-5 rel-RMS and energies
+(sums of like-signed terms) to 1e-6."""
 import numpy as np
 import pytest
 
