@@ -242,6 +242,18 @@ class _InnerLoop(torch.autograd.Function):
         return gx, gv, gs, gf, None
 
 
+def _inner_fusable(x, v, f_field, f_bond, model):
+    """Whether _InnerLoop may take these inputs.  Its kernels read and write
+    float32 (n, 3) arrays on the plan's device and check nothing: a velocity or
+    force that broadcasts, another type or a tensor elsewhere goes step by
+    step, under torch's own rules."""
+    md = model.md
+    shape, dev = (md.n, 3), md.r.device
+    return model.fused_inner and all(
+        t.is_cuda and t.dtype == torch.float32 and t.shape == shape and t.device == dev
+        for t in (x, v, f_field, f_bond))
+
+
 def field_force(x, chi, model):
     """The slow force of the outer kicks: the field force, plus the
     PIC_Spectral electrostatic force of a charged system."""
@@ -300,7 +312,7 @@ def respa_step(x, v, f_field, f_bond, chi, model, step=None):
     md = model.md
     m, dt, n_in = md.mass, md.dt, md.respa
     dto = n_in * dt
-    if model.fused_inner:
+    if _inner_fusable(x, v, f_field, f_bond, model):
         x, v, f_bond = _InnerLoop.apply(x, v, f_field, f_bond, model)
     else:
         v = v + (0.5 * dto / m) * f_field
