@@ -41,6 +41,7 @@ Scope: NVE or NVT (CSVR); no barostat in the differentiated step;
 PIC_Spectral electrostatics (not the GPE variant).
 """
 import math
+import operator
 
 import numpy as np
 import torch
@@ -360,13 +361,40 @@ class _ZProfile(torch.autograd.Function):
         return gx, None, None, None, None
 
 
+def _untransformed(x, types):
+    """Whether these are plain tensors that no vmap, torch.func transform,
+    forward-mode derivative, trace or dispatch mode follows: those need tensor
+    operations to follow."""
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and type(types) is torch.Tensor
+            and not torch._C._are_functorch_transforms_active()
+            and torch.autograd.forward_ad.unpack_dual(x).tangent is None
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0)
+
+
+def _profile_fusable(x, types, n_types, n_bins, box):
+    """Whether _ZProfile may take these inputs.  Its kernels read one int32
+    type per float32 bead and check no length; a box given as a tensor may want
+    a gradient.  Everything else takes the tensor form: types that broadcast,
+    and what torch refuses."""
+    if not (x.is_cuda and types.is_cuda and types.device == x.device
+            and x.dtype == torch.float32 and types.dtype == torch.int32
+            and x.dim() == 2 and x.shape[1] == 3 and x.shape[0] > 0
+            and types.dim() == 1 and types.shape[0] == x.shape[0]
+            and x.is_contiguous() and types.is_contiguous()):
+        return False
+    if isinstance(box, torch.Tensor) or any(isinstance(b, torch.Tensor) for b in box):
+        return False
+    return (n_types >= 1 and n_bins >= 1 and n_types * n_bins <= 2 ** 28
+            and all(0.0 < b < math.inf for b in box) and _untransformed(x, types))
+
+
 def z_profile(x, types, n_types, n_bins, box):
     """Per-type number density along z (beads / nm^3) with linear binning
     onto bin centres (periodic), differentiable in the positions."""
-    if (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and types.is_cuda
-            and types.dtype == torch.int32 and types.is_contiguous() and x.shape[0] > 0
-            and x.dim() == 2 and x.shape[1] == 3):
-        return _ZProfile.apply(x, types, n_types, n_bins, [float(b) for b in box])
+    if _profile_fusable(x, types, n_types, n_bins, box):
+        return _ZProfile.apply(x, types, operator.index(n_types), operator.index(n_bins),
+                               [float(b) for b in box])
     return _z_profile_torch(x, types, n_types, n_bins, box)
 
 
