@@ -49,6 +49,7 @@ _SIGNATURES = {
     "hpf_ctx_set_spectral_tile": [P, I],
     "hpf_ctx_get_spectral_tile": [P, ctypes.POINTER(I), ctypes.POINTER(I)],
     "hpf_ctx_set_functional": [P, ctypes.POINTER(D), ctypes.POINTER(D), D, D],
+    "hpf_ctx_set_functional_on": [P, ctypes.POINTER(D), ctypes.POINTER(D), D, D, P],
     "hpf_ctx_set_functional_chi": [P, P, I, I, D, D, D, D, P],
     "hpf_z_profile": [P, P, I64, I, I, D, D, P, P, P],
     "hpf_z_profile_vjp": [P, P, I64, I, I, D, D, P, P, P],

@@ -58,8 +58,8 @@ def functional_coefficients(kind, chi, kappa, rho0, a):
 
 
 def _set(pm, Q, b, c, sigma):
-    _lib.call("hpf_ctx_set_functional", pm._h, _lib.dvec(Q.reshape(-1)), _lib.dvec(b), float(c),
-              float(sigma))
+    _lib.call("hpf_ctx_set_functional_on", pm._h, _lib.dvec(Q.reshape(-1)), _lib.dvec(b),
+              float(c), float(sigma), _lib.stream_ptr())
     pm._functional = None  # the cached key no longer describes the context
 
 

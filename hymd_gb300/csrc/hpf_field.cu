@@ -1140,6 +1140,7 @@ int hpf_ctx_destroy(hpf_ctx* c) {
     cudaFree(c->fft_work);
     cudaFree(c->d_box);
     cudaFree(c->d_fun);
+    if (c->fun_set) cudaEventDestroy(c->fun_set);
     cudaFree(c->d_acc);
     cudaFree(c->d_grid);
     cudaFree(c->d_spec);
@@ -1195,6 +1196,7 @@ int hpf_ctx_create(hpf_ctx** out, int n0, int n1, int n2, int T, const double bo
     } while (0)
     CK(cudaMalloc(&c->d_box, sizeof(BoxState)));
     CK(cudaMalloc(&c->d_fun, sizeof(Functional)));
+    CK(cudaEventCreateWithFlags(&c->fun_set, cudaEventDisableTiming));
     CK(cudaMalloc(&c->d_acc, sizeof(unsigned long long) * (size_t)(T + 1) * c->M));
     CK(cudaMemset(c->d_acc, 0, sizeof(unsigned long long) * (size_t)(T + 1) * c->M));
     CK(cudaMalloc(&c->d_grid, sizeof(float) * (size_t)G * c->M));
@@ -1303,6 +1305,11 @@ int hpf_ctx_box_state(hpf_ctx* c, void** d_state) {
 
 int hpf_ctx_set_functional(hpf_ctx* c, const double* Q, const double* b, double cc,
                            double sigma) {
+    return hpf_ctx_set_functional_on(c, Q, b, cc, sigma, nullptr);
+}
+
+int hpf_ctx_set_functional_on(hpf_ctx* c, const double* Q, const double* b, double cc,
+                              double sigma, void* stream) {
     if (!c || !Q || !b) return HPF_ERR_ARG;
     const int T = c->T;
     for (int i = 0; i < T; ++i) {
@@ -1316,7 +1323,15 @@ int hpf_ctx_set_functional(hpf_ctx* c, const double* Q, const double* b, double 
     c->h_fun.c = cc;
     c->h_fun.sigma2_half = (float)(0.5 * sigma * sigma);
     c->h_fun.sigma2_half_d = 0.5 * sigma * sigma;
-    HPF_CUDA_TRY(cudaMemcpy(c->d_fun, &c->h_fun, sizeof(Functional), cudaMemcpyHostToDevice));
+    // after everything queued on the stream that still reads the old one, and
+    // after a functional queued from the device on whichever stream; complete
+    // when the call returns, so that every stream sees it
+    cudaStream_t st = as_stream(stream);
+    if (c->fun_queued) HPF_CUDA_TRY(cudaStreamWaitEvent(st, c->fun_set, 0));
+    HPF_CUDA_TRY(cudaMemcpyAsync(c->d_fun, &c->h_fun, sizeof(Functional), cudaMemcpyHostToDevice,
+                                 st));
+    HPF_CUDA_TRY(cudaStreamSynchronize(st));
+    c->fun_queued = false;
     return HPF_OK;
 }
 
@@ -1327,6 +1342,12 @@ int hpf_ctx_set_functional_chi(hpf_ctx* c, const void* chi, int chi_f64, int wit
         c->d_fun, c->T, with_chi && !chi_f64 ? (const float*)chi : nullptr,
         with_chi && chi_f64 ? (const double*)chi : nullptr, kappa, rho0, a, sigma);
     HPF_LAUNCH_CHECK();
+    cudaStreamCaptureStatus cap;
+    HPF_CUDA_TRY(cudaStreamIsCapturing(as_stream(stream), &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+        HPF_CUDA_TRY(cudaEventRecord(c->fun_set, as_stream(stream)));
+        c->fun_queued = true;
+    }
     return HPF_OK;
 }
 

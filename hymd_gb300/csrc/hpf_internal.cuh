@@ -46,6 +46,10 @@ struct hpf_ctx {
     BoxState h_box;           // host mirror (last value set from the host)
     Functional* d_fun;        // device
     Functional h_fun;
+    // the last functional queued from the device (hpf_ctx_set_functional_chi),
+    // when it was queued outside a capture: a host one has to come after it
+    cudaEvent_t fun_set;
+    bool fun_queued;
     unsigned long long* d_acc;  // paint accumulators int64[T+1][M] (the +1 is for charges)
     float* d_grid;            // real scratch float[3T][M] (densities / force mesh)
     float2* d_spec;           // spectral scratch float2[3T][Mc]

@@ -89,8 +89,8 @@ class ParticleMesh:
             T = self.n_types
             if Q.shape != (T, T):
                 raise ValueError(f"functional has {Q.shape[0]} types, mesh context has {T}")
-            _lib.call("hpf_ctx_set_functional", self._h, _lib.dvec(Q.reshape(-1)), _lib.dvec(b),
-                      float(c), float(sigma))
+            _lib.call("hpf_ctx_set_functional_on", self._h, _lib.dvec(Q.reshape(-1)),
+                      _lib.dvec(b), float(c), float(sigma), _lib.stream_ptr())
             self._functional = key
             self._functional_Q = Q
         return Q, b, c, sigma

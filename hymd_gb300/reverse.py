@@ -109,8 +109,8 @@ class ForceModel:
                                           self.rho0, self.a)
         key = (Q.tobytes(), b.tobytes(), c, self.sigma)
         if key != self._key:
-            _lib.call("hpf_ctx_set_functional", self.pm._h, _lib.dvec(Q.reshape(-1)),
-                      _lib.dvec(b), float(c), float(self.sigma))
+            _lib.call("hpf_ctx_set_functional_on", self.pm._h, _lib.dvec(Q.reshape(-1)),
+                      _lib.dvec(b), float(c), float(self.sigma), _lib.stream_ptr())
             self.pm._functional = None
             self._key = key
 

@@ -150,6 +150,12 @@ int hpf_ctx_get_spectral_tile(const hpf_ctx* ctx, int* width, int* allowed_mask)
  * width sigma (hymd/hamiltonian.py:74-486, H at :57-71).  Q is T*T row-major. */
 int hpf_ctx_set_functional(hpf_ctx* ctx, const double* Q, const double* b, double c,
                            double sigma);
+/* The same after the work queued on `stream` (the one above: on the legacy
+ * default stream, which non-blocking streams do not wait for).  Both wait for a
+ * functional queued by hpf_ctx_set_functional_chi, and return when theirs is in
+ * place; not under stream capture. */
+int hpf_ctx_set_functional_on(hpf_ctx* ctx, const double* Q, const double* b, double c,
+                              double sigma, void* stream);
 /* The same for the reference's functionals (hymd/hamiltonian.py:74-486) from
  * their parameters, formed on the device in stream order: chi device
  * float / double [T][T] (used symmetrised, its diagonal unused) with with_chi,
