@@ -74,7 +74,6 @@ class ForceModel:
         self.T = md.T
         self.box = md.box
         self.box_f = md.box.float()
-        self._key = None
         # the inner loop as one launch each way (hpf_respa_vjp); a molecule
         # too large for its shared memory keeps the step-by-step form
         ok = _lib.I(0)
@@ -103,16 +102,15 @@ class ForceModel:
                       int(chi.dtype == torch.float64), int(self.kind == "DefaultWithChi"),
                       self.kappa, self.rho0, a, self.sigma, _lib.stream_ptr())
             self.pm._functional = None
-            self._key = None
             return
         Q, b, c = functional_coefficients(self.kind, chi.detach().cpu().numpy(), self.kappa,
                                           self.rho0, self.a)
-        key = (Q.tobytes(), b.tobytes(), c, self.sigma)
-        if key != self._key:
+        # kept on the mesh, where whoever sets another functional replaces it
+        key = ("chi", Q.tobytes(), b.tobytes(), c, self.sigma)
+        if key != self.pm._functional:
             _lib.call("hpf_ctx_set_functional_on", self.pm._h, _lib.dvec(Q.reshape(-1)),
                       _lib.dvec(b), float(c), float(self.sigma), _lib.stream_ptr())
-            self.pm._functional = None
-            self._key = key
+            self.pm._functional = key
 
 
 class _FieldForce(torch.autograd.Function):
