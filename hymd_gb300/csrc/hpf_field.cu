@@ -1141,6 +1141,7 @@ int hpf_ctx_destroy(hpf_ctx* c) {
     cudaFree(c->d_box);
     cudaFree(c->d_fun);
     if (c->fun_set) cudaEventDestroy(c->fun_set);
+    sums_release(c->pending);
     cudaFree(c->d_acc);
     cudaFree(c->d_grid);
     cudaFree(c->d_spec);
@@ -1560,7 +1561,8 @@ int hpf_field_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
     cudaStream_t st = as_stream(stream);
     TypeScale sc;
     for (int t = 0; t < c->T; ++t) sc.s[t] = (float)type_mass[t];
-    int r;
+    int r = sums_join(c->pending, st);
+    if (r != HPF_OK) return r;
     if (c->spec_fused) {
         if ((r = do_paint(c, pos, types, nullptr, n, c->T, sc, c->d_grid, st, pos_scale,
                           false)) != HPF_OK)
@@ -1730,13 +1732,9 @@ int hpf_field_pic_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
     cudaStream_t st = as_stream(stream);
     // rRESPA sums still running beside this call, joined before the k-space
     // pass; at once where the deposits are still to be made or both chains run
-    cudaEvent_t join = c->pending;
-    c->pending = nullptr;
-    if (join && (!painted || charges || !c->spec_fused)) {
-        HPF_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
-        join = nullptr;
-    }
     int r;
+    if ((!painted || charges || !c->spec_fused) && (r = sums_join(c->pending, st)) != HPF_OK)
+        return r;
     if (!c->spec_fused) {
         // the library-FFT path shares its plans' work area: one chain after
         // the other.  Density deposits made elsewhere are finalised here;
@@ -1768,7 +1766,7 @@ int hpf_field_pic_step(hpf_ctx* c, float* pos, const int32_t* types, int64_t n,
         if (!painted && (r = do_paint(c, pos, types, nullptr, n, c->T, sc, c->d_grid, st,
                                       pos_scale, false)) != HPF_OK)
             return r;
-        if ((r = spectral_field_force(c, sc.s, sums, st, join)) != HPF_OK) return r;
+        if ((r = spectral_field_force(c, sc.s, sums, st, c->pending)) != HPF_OK) return r;
         if (n > 0)
             return launch_readout(c, c->d_grid, pos, types, nullptr, n, c->T, force, kick, st,
                                   pos_w, rscale);

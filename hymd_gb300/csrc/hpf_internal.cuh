@@ -38,6 +38,22 @@ struct Functional {
     float pad;
 };
 
+// Completion of a plan's deferred sums.  Held by the plan and by the mesh
+// context that is to join them, either of which may be destroyed first.  A step
+// that fails between the two leaves `open`, and whichever call comes next on
+// the plan or the context joins them.
+struct SumsEvent {
+    cudaEvent_t done;
+    int refs;
+    bool open;                   // recorded, and not yet waited for
+    unsigned long long capture;  // the capture it was recorded in (0: none)
+};
+void sums_release(SumsEvent* s);
+// st waits for the sums if they are open (s may be NULL).
+int sums_join(SumsEvent* s, cudaStream_t st);
+// Id of the capture st is in, 0 outside one.
+int capture_id(cudaStream_t st, unsigned long long* id);
+
 struct hpf_ctx {
     int n0, n1, n2, T;
     int64_t M, Mc;
@@ -103,10 +119,9 @@ struct hpf_ctx {
     double* pic_spec_ws;
     cudaStream_t pic_stream;
     cudaEvent_t pic_fork, pic_join;
-    // the rRESPA sums still running on their plan's second stream
-    // (hpf_respa_plan_defer): the field step waits for this event before its
-    // k-space pass, then forgets it.  Owned by the plan.
-    cudaEvent_t pending;
+    // rRESPA sums still running on their plan's second stream
+    // (hpf_respa_plan_defer), which the field step joins before its k-space pass
+    SumsEvent* pending;
 };
 
 // Buffers of one chain of the fused spectral passes: spectra in (pass A ->
@@ -146,9 +161,9 @@ bool spectral_eligible(const hpf_ctx* c);
 int spectral_setup(hpf_ctx* c);
 bool spectral_tile_ok(const hpf_ctx* c, int W);
 int spectral_set_tile(hpf_ctx* c, int W);
-// join (may be NULL): an event that the pass after A waits for.
+// join (may be NULL): sums that the pass after A waits for.
 int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st,
-                         cudaEvent_t join = nullptr);
+                         SumsEvent* join = nullptr);
 // real_in non-NULL: the input is that real grid (float[M]) instead of the
 // charge accumulator; filter = false drops H(k) from the Poisson map (the GPE
 // solve's psi = scale (q + pol) / k^2).

@@ -72,9 +72,10 @@ struct hpf_respa_plan {
     cudaStream_t free_stream;
     cudaEvent_t free_fork, free_join;
     // hpf_respa_plan_defer: the sums run on free_stream after both kernels
-    // (sums_fork) and are joined by the field step (sums_done)
+    // (sums_fork) and are joined by the field step (sums)
     int defer;
-    cudaEvent_t sums_fork, sums_done;
+    cudaEvent_t sums_fork;
+    SumsEvent* sums;
 };
 
 namespace {
@@ -1035,12 +1036,55 @@ size_t vjp_smem(const hpf_respa_plan* p) {
     return (p->smem_group + sizeof(float4) * p->mx_beads) * (p->warp_mode ? kWarps : 1);
 }
 
+SumsEvent* new_sums() {
+    SumsEvent* s = new SumsEvent();
+    s->refs = 1;
+    if (cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming) == cudaSuccess) return s;
+    delete s;
+    return nullptr;
+}
+
 int grid_size(const hpf_respa_plan* p) {
     const int g = p->warp_mode ? (p->n_groups + kWarps - 1) / kWarps : p->n_groups;
     return g + p->n_free_blocks;
 }
 
 }  // namespace
+
+void sums_release(SumsEvent* s) {
+    if (!s || --s->refs > 0) return;
+    cudaEventDestroy(s->done);
+    delete s;
+}
+
+int capture_id(cudaStream_t st, unsigned long long* id) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    *id = 0;
+    HPF_CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, id));
+    if (cs != cudaStreamCaptureStatusActive) *id = 0;
+    return HPF_OK;
+}
+
+int sums_join(SumsEvent* s, cudaStream_t st) {
+    if (!s || !s->open) return HPF_OK;
+    unsigned long long id = 0;
+    int r = capture_id(st, &id);
+    if (r != HPF_OK) return r;
+    if (id == s->capture) {
+        HPF_CUDA_TRY(cudaStreamWaitEvent(st, s->done, 0));
+    } else if (s->capture == 0) {
+        // left by a failed step before this capture began: no part of the
+        // graph, so the host waits for them here (one short block)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        HPF_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaEventSynchronize(s->done);
+        HPF_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+        HPF_CUDA_TRY(e);
+    }
+    // (else recorded in a capture that has ended: nothing runs)
+    s->open = false;
+    return HPF_OK;
+}
 
 extern "C" {
 
@@ -1092,7 +1136,7 @@ int hpf_respa_plan_destroy(hpf_respa_plan* p) {
     if (p->free_fork) cudaEventDestroy(p->free_fork);
     if (p->free_join) cudaEventDestroy(p->free_join);
     if (p->sums_fork) cudaEventDestroy(p->sums_fork);
-    if (p->sums_done) cudaEventDestroy(p->sums_done);
+    sums_release(p->sums);
     delete p;
     return HPF_OK;
 }
@@ -1356,7 +1400,7 @@ int hpf_respa_plan_create(hpf_respa_plan** out, int64_t n, int64_t nb, const int
     if (cudaMalloc(&p->partials, sizeof(double) * kOut * (size_t)std::max(grid, 1)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&p->free_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->sums_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&p->sums_done, cudaEventDisableTiming) != cudaSuccess ||
+        !(p->sums = new_sums()) ||
         cudaEventCreateWithFlags(&p->free_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->free_join, cudaEventDisableTiming) != cudaSuccess) {
         hpf_respa_plan_destroy(p);
@@ -1432,6 +1476,10 @@ int respa_run(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
     const int grid = grid_size(p);
     if (grid == 0) return HPF_OK;
     cudaStream_t st = as_stream(stream);
+    // deferred sums that no field step has joined still read the partials
+    int rj = sums_join(p->sums, st);
+    if (rj == HPF_OK && field_ctx) rj = sums_join(field_ctx->pending, st);
+    if (rj != HPF_OK) return rj;
     const float h_out = (float)(0.5 * respa_inner * dt), hdt = (float)(0.5 * dt);
     PaintFuse pfv;
     memset(&pfv, 0, sizeof(pfv));
@@ -1490,13 +1538,20 @@ int respa_run(hpf_respa_plan* p, float* r, float* v, float* f_bonded,
     if (out && pf && p->defer && !baro) {
         // the sums (one block, a latency chain) beside the field step's first
         // pass instead of before it
+        SumsEvent* s = p->sums;
         HPF_CUDA_TRY(cudaEventRecord(p->sums_fork, st));
         HPF_CUDA_TRY(cudaStreamWaitEvent(p->free_stream, p->sums_fork, 0));
         const cudaError_t e =
             launch_pdl(k_respa_finish, 1, kFinishThreads, 0, p->free_stream,
                        static_cast<const double*>(p->partials), G, out, bf, d_err);
-        HPF_CUDA_TRY(cudaEventRecord(p->sums_done, p->free_stream));
-        field_ctx->pending = p->sums_done;
+        HPF_CUDA_TRY(cudaEventRecord(s->done, p->free_stream));
+        s->open = true;
+        if ((rj = capture_id(st, &s->capture)) != HPF_OK) return rj;
+        if (field_ctx->pending != s) {
+            sums_release(field_ctx->pending);
+            field_ctx->pending = s;
+            ++s->refs;
+        }
         return e == cudaSuccess ? HPF_OK : HPF_ERR_CUDA;
     }
     if (out && launch_pdl(k_respa_finish, 1, kFinishThreads, 0, st,
@@ -1593,6 +1648,8 @@ int hpf_respa_forces(hpf_respa_plan* p, const float* r, float* f_bonded, const d
     const int grid = p->warp_mode ? (p->n_groups + kWarps - 1) / kWarps : p->n_groups;
     if (grid == 0) return HPF_OK;
     cudaStream_t st = as_stream(stream);
+    const int rj = sums_join(p->sums, st);
+    if (rj != HPF_OK) return rj;
     SlowForces sf;
     sf.n = 0;
     // v is neither read nor written in this mode; r is only read

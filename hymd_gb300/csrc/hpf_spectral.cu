@@ -851,7 +851,7 @@ size_t spectral_ws_words(const hpf_ctx* c) { return 4 * (size_t)c->spec_max_tile
 // accumulators (T grids, painted) -> force mesh c->d_grid [3T][M]; sums as
 // k_kspace_force's (out[0..3]) when non-null.
 int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cudaStream_t st,
-                         cudaEvent_t join) {
+                         SumsEvent* join) {
     SpecGeom g = spec_geom(c, c->spec_W);
     g.inplace = tile_inplace(c, g.W);
     SpecScale sc;
@@ -864,10 +864,11 @@ int spectral_field_force(hpf_ctx* c, const float* type_scale, double* sums, cuda
                        : HPF_ERR_CUDA;
         }) != HPF_OK)
         return HPF_ERR_CUDA;
-    if (join) HPF_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
+    int r = sums_join(join, st);
+    if (r != HPF_OK) return r;
     double* part = c->d_spec_ws;
     unsigned int* tick = reinterpret_cast<unsigned int*>(c->d_spec_ws + 4 * (size_t)c->spec_max_tiles);
-    int r = with_kspace(c->n0, [&](auto kd, auto, auto) {
+    r = with_kspace(c->n0, [&](auto kd, auto, auto) {
         return launch_pdl(kd, c->spec_tiles, kSpecThreads, ts, st, c->d_spec_phi, c->d_spec, g,
                           c->T, c->d_box, c->d_fun, c->d_tw, sums, part, tick, nullptr) == cudaSuccess
                    ? HPF_OK

@@ -499,7 +499,9 @@ int hpf_respa_plan_info(const hpf_respa_plan* plan, int* n_mol_blocks, int* n_fr
  * beside the calls that follow on `stream`, and the next hpf_field_pic_step on
  * its field_ctx, which must follow on the same stream, waits for them; on = 0
  * (the default), and always with a barostat: complete in stream order when the
- * call returns. */
+ * call returns.  Where another step, force evaluation or hpf_field_step on the
+ * plan or field_ctx comes instead, that one waits for them; plan and field_ctx
+ * may be destroyed in either order in between. */
 int hpf_respa_plan_defer(hpf_respa_plan* plan, int on);
 /* hpf_respa_step (the launch itself) is declared after the barostat
  * arguments below. */
