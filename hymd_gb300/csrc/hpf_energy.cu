@@ -386,9 +386,14 @@ size_t x_smem(int n0, int G, int W, int* ts) {
 
 }  // namespace
 
-// Twiddles (double-float) and the reduction scratch, on first use.
-int energy_df_setup(hpf_ctx* c) {
+// Twiddles (double-float) and the reduction scratch, on first use, filled in
+// the stream of the call that needs them (refused under stream capture, where
+// nothing may be allocated).
+int energy_df_setup(hpf_ctx* c, cudaStream_t st) {
     if (c->df_tw) return HPF_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+        return HPF_ERR_ARG;
     using hpf_fft::kTable2;
     using hpf_fft::kTable3;
     float4 h[kTable2 + kTable3];
@@ -403,8 +408,9 @@ int energy_df_setup(hpf_ctx* c) {
                          sizeof(float4) * (size_t)(c->n0 + c->n1 + c->n2 / 2 + 1);
     float4* tw = nullptr;
     HPF_CUDA_TRY(cudaMalloc(&tw, sizeof(h) + bytes));
-    if (cudaMemcpy(tw, h, sizeof(h), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(reinterpret_cast<char*>(tw) + sizeof(h), 0, bytes) != cudaSuccess) {
+    // (h is pageable: copied from before the call returns)
+    if (cudaMemcpyAsync(tw, h, sizeof(h), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemsetAsync(reinterpret_cast<char*>(tw) + sizeof(h), 0, bytes, st) != cudaSuccess) {
         cudaFree(tw);
         return HPF_ERR_CUDA;
     }

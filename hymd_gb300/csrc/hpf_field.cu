@@ -1082,7 +1082,7 @@ int pic_chain_setup(hpf_ctx* c, cudaStream_t st) {
         cudaMalloc(&c->pic_spec, sizeof(float2) * 2 * (size_t)c->Mc) != cudaSuccess ||
         cudaMalloc(&c->pic_grid, sizeof(float) * 4 * (size_t)c->M) != cudaSuccess ||
         cudaMalloc(&c->pic_spec_ws, sizeof(double) * words) != cudaSuccess ||
-        cudaMemset(c->pic_spec_ws, 0, sizeof(double) * words) != cudaSuccess ||
+        cudaMemsetAsync(c->pic_spec_ws, 0, sizeof(double) * words, st) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->pic_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->pic_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->pic_stream, cudaStreamNonBlocking) != cudaSuccess)
@@ -1502,7 +1502,7 @@ int hpf_energy_fp64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t 
     const int T = c->T;
     if (energy_df_ok(c)) {
         int r;
-        if ((r = ensure_spec64(c)) != HPF_OK || (r = energy_df_setup(c)) != HPF_OK ||
+        if ((r = energy_df_setup(c, st)) != HPF_OK || (r = ensure_spec64(c)) != HPF_OK ||
             (r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK)
             return r;
         return energy_df(c, charges ? T + 1 : T, type_mass, type_charges,
@@ -2188,12 +2188,12 @@ __global__ void k_gpe_loop_init(int* it, unsigned int* max_bits, cudaGraphCondit
     cudaGraphSetConditional(h, run ? 1u : 0u);
 }
 
-int gpe_scratch(hpf_ctx* c) {
+int gpe_scratch(hpf_ctx* c, cudaStream_t st) {
     if (c->gpe_grid) return HPF_OK;
     HPF_CUDA_TRY(cudaMalloc(&c->gpe_grid, sizeof(float) * (size_t)kGpeGrids * c->M));
     HPF_CUDA_TRY(cudaMalloc(&c->gpe_spec, sizeof(float2) * (size_t)4 * c->Mc));
     HPF_CUDA_TRY(cudaMalloc(&c->gpe_ws, sizeof(double) * HPF_OUT_DOUBLES));
-    HPF_CUDA_TRY(cudaMemset(c->gpe_ws, 0, sizeof(double) * HPF_OUT_DOUBLES));
+    HPF_CUDA_TRY(cudaMemsetAsync(c->gpe_ws, 0, sizeof(double) * HPF_OUT_DOUBLES, st));
     HPF_CUDA_TRY(cudaMallocHost(&c->gpe_host, sizeof(double) * 2));
     return HPF_OK;
 }
@@ -2322,7 +2322,7 @@ extern "C" int hpf_gpe_step(hpf_ctx* c, const float* pos, const int32_t* types,
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
         return HPF_ERR_ARG;
-    int r = gpe_scratch(c);
+    int r = gpe_scratch(c, st);
     if (r != HPF_OK) return r;
     const int T = c->T;
     const int64_t M = c->M, Mc = c->Mc;

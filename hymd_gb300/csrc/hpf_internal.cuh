@@ -183,7 +183,7 @@ int spectral_fields(hpf_ctx* c, const float* type_scale, float* phi, float2* phi
 // FP64 energy sums in double-float arithmetic (hpf_energy.cu): whether they
 // apply, setup on first use, painted accumulators (G grids) -> out[32].
 bool energy_df_ok(const hpf_ctx* c);
-int energy_df_setup(hpf_ctx* c);
+int energy_df_setup(hpf_ctx* c, cudaStream_t st);
 int energy_df(hpf_ctx* c, int G, const double* type_mass, const double* type_charges,
               double four_pi_fac, float4* spec, double* out, cudaStream_t st);
 // words of a pass-B partial-sum buffer (partials of the narrowest tile + ticket)
