@@ -387,13 +387,9 @@ size_t x_smem(int n0, int G, int W, int* ts) {
 }  // namespace
 
 // Twiddles (double-float) and the reduction scratch, on first use, filled in
-// the stream of the call that needs them (refused under stream capture, where
-// nothing may be allocated).
+// the stream of the call that needs them (never under capture).
 int energy_df_setup(hpf_ctx* c, cudaStream_t st) {
     if (c->df_tw) return HPF_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
-        return HPF_ERR_ARG;
     using hpf_fft::kTable2;
     using hpf_fft::kTable3;
     float4 h[kTable2 + kTable3];

@@ -858,24 +858,40 @@ int ensure_spec64(hpf_ctx* c) {
 }
 
 // The FP64 buffers and the D2Z plans (T densities, T + 1 with the charges)
-// are only needed for energies and gradients: created on first use.
-int ensure_d2z(hpf_ctx* c, int q) {
-    if (c->has_d2z[q]) return HPF_OK;
+// are only needed for energies and gradients: created on first use, both at
+// once, so that a later call with the other may be captured.
+int ensure_d2z(hpf_ctx* c) {
     const int T = c->T;
     if (!c->d_grid64)
         HPF_CUDA_TRY(cudaMalloc(&c->d_grid64, sizeof(double) * (size_t)(T + 1) * c->M));
     int r = ensure_spec64(c);
-    if (r != HPF_OK) return r;
-    long long nn[3] = {c->n0, c->n1, c->n2};
-    size_t ws = 0;
-    if (cufftCreate(&c->plan_d2z[q]) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
-    if (cufftMakePlanMany64(c->plan_d2z[q], 3, nn, NULL, 1, c->M, NULL, 1, c->Mc, CUFFT_D2Z, T + q,
-                            &ws) != CUFFT_SUCCESS) {
-        cufftDestroy(c->plan_d2z[q]);
-        return HPF_ERR_CUFFT;
+    for (int q = 0; q < 2 && r == HPF_OK; ++q) {
+        if (c->has_d2z[q]) continue;
+        long long nn[3] = {c->n0, c->n1, c->n2};
+        size_t ws = 0;
+        if (cufftCreate(&c->plan_d2z[q]) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
+        if (cufftMakePlanMany64(c->plan_d2z[q], 3, nn, NULL, 1, c->M, NULL, 1, c->Mc, CUFFT_D2Z,
+                                T + q, &ws) != CUFFT_SUCCESS) {
+            cufftDestroy(c->plan_d2z[q]);
+            return HPF_ERR_CUFFT;
+        }
+        c->has_d2z[q] = true;
     }
-    c->has_d2z[q] = true;
-    return HPF_OK;
+    return r;
+}
+
+// What an energy on the context's present path needs.  Nothing may be
+// allocated under capture: where something is missing, the call is refused
+// before it touches the device.
+int energy_setup(hpf_ctx* c, cudaStream_t st) {
+    const bool df = energy_df_ok(c);
+    if (df ? c->df_tw && c->d_spec64 : c->has_d2z[0] && c->has_d2z[1]) return HPF_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+        return HPF_ERR_ARG;
+    if (!df) return ensure_d2z(c);
+    const int r = energy_df_setup(c, st);
+    return r != HPF_OK ? r : ensure_spec64(c);
 }
 
 // Deposits of the densities, and of the charges into slot T when given.
@@ -899,8 +915,7 @@ int paint_f64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n, con
 int density_spectra_f64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t n,
                         const double* type_mass, const float* charges, cudaStream_t st) {
     const int q = charges ? 1 : 0;
-    int r = ensure_d2z(c, q);
-    if (r != HPF_OK) return r;
+    int r;
     const int T = c->T;
     TypeScaleD sc;
     for (int t = 0; t < T; ++t) sc.s[t] = type_mass[t];
@@ -1270,6 +1285,15 @@ int hpf_ctx_set_spectral(hpf_ctx* c, int fused) {
     if (!c || fused < 0 || fused > 1) return HPF_ERR_ARG;
     if (fused && !c->spec_ok) return HPF_ERR_ARG;
     c->spec_fused = fused;
+    if (!c->d_spec64) return HPF_OK;
+    // energies have been evaluated on the other path: those of this one may be
+    // captured next, so they are made ready here (in relaxed mode, should
+    // something be captured meanwhile); what fails is reported by the energy
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    HPF_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    if (energy_setup(c, nullptr) != HPF_OK || cudaStreamSynchronize(nullptr) != cudaSuccess)
+        cudaGetLastError();
+    HPF_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
     return HPF_OK;
 }
 
@@ -1500,16 +1524,16 @@ int hpf_energy_fp64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t 
     if (!c || !type_mass || !out || n < 0 || (n > 0 && (!pos || !types))) return HPF_ERR_ARG;
     cudaStream_t st = as_stream(stream);
     const int T = c->T;
+    int r0 = energy_setup(c, st);
+    if (r0 != HPF_OK) return r0;
     if (energy_df_ok(c)) {
         int r;
-        if ((r = energy_df_setup(c, st)) != HPF_OK || (r = ensure_spec64(c)) != HPF_OK ||
-            (r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK)
-            return r;
+        if ((r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK) return r;
         return energy_df(c, charges ? T + 1 : T, type_mass, type_charges,
                          4.0 * 3.14159265358979323846 * elec_factor,
                          reinterpret_cast<float4*>(c->d_spec64), out, st);
     }
-    int r0 = density_spectra_f64(c, pos, types, n, type_mass, charges, st);
+    r0 = density_spectra_f64(c, pos, types, n, type_mass, charges, st);
     if (r0 != HPF_OK) return r0;
     TypeScaleD qt;
     for (int t = 0; t < T; ++t) qt.s[t] = type_charges ? type_charges[t] : 0.0;
