@@ -2279,7 +2279,8 @@ int gpe_update(hpf_ctx* c, float* pol, int kind, float w, const GpeLoop& l, cuda
 // not run executes no iteration.
 int gpe_loop_graph(hpf_ctx* c, float* pol, int kind, double mixing, double crit, int max_iter) {
     if (c->gpe_exec && c->gpe_key_pol == pol && c->gpe_key_kind == kind &&
-        c->gpe_key_mix == mixing && c->gpe_key_crit == crit && c->gpe_key_max == max_iter)
+        c->gpe_key_mix == mixing && c->gpe_key_crit == crit && c->gpe_key_max == max_iter &&
+        c->gpe_key_fused == c->spec_fused)
         return HPF_OK;
     if (c->gpe_exec) cudaGraphExecDestroy(c->gpe_exec);
     if (c->gpe_graph) cudaGraphDestroy(c->gpe_graph);
@@ -2325,6 +2326,7 @@ int gpe_loop_graph(hpf_ctx* c, float* pol, int kind, double mixing, double crit,
     c->gpe_key_mix = mixing;
     c->gpe_key_crit = crit;
     c->gpe_key_max = max_iter;
+    c->gpe_key_fused = c->spec_fused;
     return HPF_OK;
 }
 

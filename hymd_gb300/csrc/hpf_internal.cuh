@@ -93,13 +93,14 @@ struct hpf_ctx {
     // the polarisation iteration as a CUDA graph: a while node whose body
     // (r2c, field map, 3 c2r, update, convergence test) sets its own
     // condition on the device; built on first use on gpe_cap, rebuilt when
-    // the iterated grid, mixing, tolerance, measure or iteration cap change
+    // the iterated grid, mixing, tolerance, measure, iteration cap or spectral
+    // path change
     cudaGraph_t gpe_graph;
     cudaGraphExec_t gpe_exec;
     cudaStream_t gpe_cap;
     const float* gpe_key_pol;
     double gpe_key_mix, gpe_key_crit;
-    int gpe_key_kind, gpe_key_max;
+    int gpe_key_kind, gpe_key_max, gpe_key_fused;
     // fused spectral passes: twiddle tables exp(-2 pi i m / 512) and
     // exp(-2 pi i m / 768), k-space tile width, partial sums + ticket
     float2* d_tw;

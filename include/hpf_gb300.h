@@ -292,9 +292,9 @@ int hpf_dihedral_hvp(float* out, const float* r, const float* lam, int64_t n, co
  * iteration runs as a CUDA graph whose while node repeats the update while
  * the convergence test, evaluated on the device after each update, holds;
  * the graph is built on the first call and again when pol_prev, mixing,
- * conv_crit, conv_kind or max_iter change.  With iterations != NULL the call
- * synchronises the stream once, at its end, and *iterations receives their
- * number.  Not capturable: a stream under capture returns HPF_ERR_ARG. */
+ * conv_crit, conv_kind, max_iter or the spectral path change.  With iterations
+ * != NULL the call synchronises the stream once, at its end, and *iterations
+ * receives their number.  Not capturable: a stream under capture returns HPF_ERR_ARG. */
 int hpf_gpe_step(hpf_ctx* ctx, const float* pos, const int32_t* types, const float* charges,
                  int64_t n, const float* phi_tilde, const double* eps_type,
                  const double* type_charges, double coulomb_constant, double conv_crit,
