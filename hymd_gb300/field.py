@@ -14,6 +14,8 @@ serve all types; functions here accept only such stacks (ValueError otherwise).
 `layouts` / `layout_q` arguments (pmesh domain layouts) are accepted and
 ignored: one GPU holds the whole system.
 """
+import math
+
 import numpy as np
 import torch
 
@@ -175,9 +177,21 @@ class _DevicePtrArray:
             self.tensor = torch.as_tensor(self, device=device)
 
 
+def _flat(lst):
+    out = []
+    for x in lst:
+        if isinstance(x, (list, tuple)):
+            out.extend(_flat(x))
+        else:
+            out.append(x)
+    return out
+
+
 def _stack_base(lst, lead_shape, dtype, name):
     """Return the stacked tensor that the list elements are views of."""
-    flat = [y for x in lst for y in (x if isinstance(x, (list, tuple)) else (x,))]
+    flat = _flat(lst)
+    if len(flat) != math.prod(lead_shape):
+        raise ValueError(f"{name} must hold {math.prod(lead_shape)} grids, got {len(flat)}")
     first = flat[0]
     _lib.require_cuda(first, name + "[0]", dtype)
     p, per = first.data_ptr(), first.numel() * first.element_size()
