@@ -14,7 +14,9 @@ serve all types; functions here accept only such stacks (ValueError otherwise).
 `layouts` / `layout_q` arguments (pmesh domain layouts) are accepted and
 ignored: one GPU holds the whole system.
 """
+import functools
 import math
+import weakref
 
 import numpy as np
 import torch
@@ -23,7 +25,7 @@ from . import _lib
 from .hamiltonian import quadratic_form
 
 _REGISTRY = {}
-_REGISTRY_FOURIER = {}
+_REGISTRY_FOURIER = weakref.WeakValueDictionary()  # (_REGISTRY holds the meshes)
 
 
 class ParticleMesh:
@@ -63,6 +65,16 @@ class ParticleMesh:
     def complex_field(self, *lead):
         return torch.zeros(*lead, self.Nmesh[0], self.Nmesh[1], self.Nmesh[2] // 2 + 1,
                            dtype=torch.complex64, device=self.device)
+
+    @functools.cached_property
+    def spec_raw(self):
+        """Spectra of the densities, for callers of hpf_r2c and its like."""
+        return self.complex_field(self.n_types)
+
+    @functools.cached_property
+    def spec_force(self):
+        """Spectra of the force mesh, for callers of hpf_kspace_force and its like."""
+        return self.complex_field(3 * self.n_types)
 
     def create(self, kind, value=0.0):
         """pmesh-style single field."""
