@@ -884,13 +884,13 @@ int ensure_d2z(hpf_ctx* c) {
 // allocated under capture: where something is missing, the call is refused
 // before it touches the device.
 int energy_setup(hpf_ctx* c, cudaStream_t st) {
-    const bool df = energy_df_ok(c);
-    if (df ? c->df_tw && c->d_spec64 : c->has_d2z[0] && c->has_d2z[1]) return HPF_OK;
+    const bool fused = energy_fused_ok(c);
+    if (fused ? c->e64_tw && c->d_spec64 : c->has_d2z[0] && c->has_d2z[1]) return HPF_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
         return HPF_ERR_ARG;
-    if (!df) return ensure_d2z(c);
-    const int r = energy_df_setup(c, st);
+    if (!fused) return ensure_d2z(c);
+    const int r = energy_fused_setup(c, st);
     return r != HPF_OK ? r : ensure_spec64(c);
 }
 
@@ -1175,7 +1175,7 @@ int hpf_ctx_destroy(hpf_ctx* c) {
     if (c->gpe_graph) cudaGraphDestroy(c->gpe_graph);
     if (c->gpe_cap) cudaStreamDestroy(c->gpe_cap);
     cudaFree(c->d_tw);
-    cudaFree(c->df_tw);
+    cudaFree(c->e64_tw);
     cudaFree(c->d_spec_ws);
     cudaFree(c->pic_spec_phi);
     cudaFree(c->pic_spec);
@@ -1526,12 +1526,11 @@ int hpf_energy_fp64(hpf_ctx* c, const float* pos, const int32_t* types, int64_t 
     const int T = c->T;
     int r0 = energy_setup(c, st);
     if (r0 != HPF_OK) return r0;
-    if (energy_df_ok(c)) {
+    if (energy_fused_ok(c)) {
         int r;
         if ((r = paint_f64(c, pos, types, n, charges, st)) != HPF_OK) return r;
-        return energy_df(c, charges ? T + 1 : T, type_mass, type_charges,
-                         4.0 * 3.14159265358979323846 * elec_factor,
-                         reinterpret_cast<float4*>(c->d_spec64), out, st);
+        return energy_fused(c, charges ? T + 1 : T, type_mass, type_charges,
+                            4.0 * 3.14159265358979323846 * elec_factor, c->d_spec64, out, st);
     }
     r0 = density_spectra_f64(c, pos, types, n, type_mass, charges, st);
     if (r0 != HPF_OK) return r0;

@@ -104,7 +104,7 @@ struct hpf_ctx {
     // fused spectral passes: twiddle tables exp(-2 pi i m / 512) and
     // exp(-2 pi i m / 768), k-space tile width, partial sums + ticket
     float2* d_tw;
-    float4* df_tw;  // double-float twiddles and scratch (energy_df_setup)
+    double2* e64_tw;  // FP64 twiddles and scratch (energy_fused_setup)
     double* d_spec_ws;
     int spec_W, spec_tiles, spec_max_tiles;
     int spec_W_pic, spec_tiles_pic;  // the charge k-space pass's own tile width
@@ -181,12 +181,12 @@ int spectral_map(hpf_ctx* c, const SpecBufs& b, const float* real_in, int grids,
 bool spectral_fields_ok(const hpf_ctx* c);
 int spectral_fields(hpf_ctx* c, const float* type_scale, float* phi, float2* phi_k, float* force,
                     float* vext, cudaStream_t st);
-// FP64 energy sums in double-float arithmetic (hpf_energy.cu): whether they
-// apply, setup on first use, painted accumulators (G grids) -> out[32].
-bool energy_df_ok(const hpf_ctx* c);
-int energy_df_setup(hpf_ctx* c, cudaStream_t st);
-int energy_df(hpf_ctx* c, int G, const double* type_mass, const double* type_charges,
-              double four_pi_fac, float4* spec, double* out, cudaStream_t st);
+// FP64 energy sums on the fused meshes (hpf_energy.cu): whether they apply,
+// setup on first use, painted accumulators (G grids) -> out[32].
+bool energy_fused_ok(const hpf_ctx* c);
+int energy_fused_setup(hpf_ctx* c, cudaStream_t st);
+int energy_fused(hpf_ctx* c, int G, const double* type_mass, const double* type_charges,
+                 double four_pi_fac, double2* spec, double* out, cudaStream_t st);
 // words of a pass-B partial-sum buffer (partials of the narrowest tile + ticket)
 size_t spectral_ws_words(const hpf_ctx* c);
 

@@ -207,8 +207,9 @@ int hpf_kspace_sums(hpf_ctx* ctx, const void* phi_fourier, const void* psi_k,
 /* FP64 energies and pressure sums of the current positions (the quantities
  * of compute_field_and_kinetic_energy, hymd/field.py:619-703, and of
  * comp_pressure, hymd/pressure.py:84-121).  The fixed-point densities (and,
- * when charges != NULL, the charge density) are converted to double grids,
- * transformed by an FP64 cuFFT and reduced in FP64 over the half spectrum.
+ * when charges != NULL, the charge density) are transformed and reduced over
+ * the half spectrum in FP64: by this library's passes on the fused meshes with
+ * up to 8 types, by an FP64 cuFFT elsewhere.
  * out: device double[32]:
  *   out[0]    A   = sum_{k!=0} w_k sum_ij Q_ij Re(phi~_i conj phi~_j)
  *   out[1+d]  B_d = sum_{k!=0} w_k k_d^2 (same)
@@ -216,8 +217,8 @@ int hpf_kspace_sums(hpf_ctx* ctx, const void* phi_fourier, const void* psi_k,
  *   out[5]    sum_k w_k sum_t q_t Re(psi_k conj phi~_t)   (type_charges q_t)
  *   out[6+d]  the same weighted by k_d^2
  *   out[16+t] mean of phi_t
- * so that W = V w(mean phi) + V/2 A.  Allocates its FP64 buffers and plan
- * on first use (not capturable then). */
+ * so that W = V w(mean phi) + V/2 A.  Allocates its FP64 buffers and plans
+ * on first use (HPF_ERR_ARG under capture then). */
 int hpf_energy_fp64(hpf_ctx* ctx, const float* pos, const int32_t* types, int64_t n,
                     const double* type_mass, const float* charges, const double* type_charges,
                     double elec_factor, double* out, void* stream);
