@@ -359,11 +359,15 @@ class _ZProfile(torch.autograd.Function):
         return gx, None, None, None, None
 
 
+def _plain(x, types):
+    return type(x) in (torch.Tensor, torch.nn.Parameter) and type(types) is torch.Tensor
+
+
 def _untransformed(x, types):
-    """Whether these are plain tensors that no vmap, torch.func transform,
-    forward-mode derivative, trace or dispatch mode follows: those need tensor
-    operations to follow."""
-    return (type(x) in (torch.Tensor, torch.nn.Parameter) and type(types) is torch.Tensor
+    """Whether these are plain tensors, on the device that kernels are launched
+    on, that no vmap, torch.func transform, forward-mode derivative, trace or
+    dispatch mode follows: those need tensor operations to follow."""
+    return (_plain(x, types) and not (x.is_cuda and x.device.index != torch.cuda.current_device())
             and not torch._C._are_functorch_transforms_active()
             and torch.autograd.forward_ad.unpack_dual(x).tangent is None
             and not torch.jit.is_tracing() and not torch.compiler.is_compiling()

@@ -253,3 +253,20 @@ def test_profile_second_derivative():
     p = z_profile(x, one, 1, bins, box)
     want = z_profile(x, one.expand(n).contiguous(), 1, bins, box)
     assert float((p - want).abs().max()) <= 1e-5 * float(want.max())
+
+
+def test_profile_on_another_device(monkeypatch):
+    """The kernels are launched on the current device: tensors of another one take the
+    tensor form, which follows them there."""
+    from hymd_gb300 import reverse
+
+    class Cuda(torch.Tensor):
+        is_cuda = True
+        device = torch.device("cuda", 1)
+
+    x = torch.rand(N, 3).as_subclass(Cuda)
+    t = torch.zeros(N, dtype=torch.int32).as_subclass(Cuda)
+    monkeypatch.setattr(reverse, "_plain", lambda *a: True)
+    for current, want in ((0, False), (1, True)):
+        monkeypatch.setattr(torch.cuda, "current_device", lambda: current)
+        assert reverse._untransformed(x, t) is want
