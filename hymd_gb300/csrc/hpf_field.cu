@@ -1021,7 +1021,7 @@ int launch_readout(hpf_ctx* c, const float* fm, const float* pos, const int32_t*
             kd.counter = kick->counter;
             kd.state = kick->state;
             kd.ws = kick->ws;
-            mode = kick->defer ? 3 : 2;
+            mode = kick->defer == 1 ? 3 : 2;
         }
     }
     if ((pos_w != nullptr) != (scale != nullptr) || (pos_w && mode == 1)) return HPF_ERR_ARG;

@@ -96,14 +96,14 @@ typedef struct {
  * this readout produces.  With thermo != NULL the same pass accumulates the
  * per-group velocity sums and the grid's last block forms the CSVR scale
  * factors (as hpf_csvr does, without applying them: call hpf_csvr_scale).
- * With defer != 0 the pass leaves the sums' block partials in ws instead, and
+ * With defer == 1 the pass leaves the sums' block partials in ws instead, and
  * hpf_csvr_apply(v, ..., the same n and ws) forms the factors and applies
  * them. */
 typedef struct {
     float* v;
     const float* prev[4];
     int n_prev;
-    int defer;
+    int defer; /* (any value but 1: not deferred) */
     double mass, dt_outer;
     const HpfCsvrArgs* thermo;
     const int32_t* group;
