@@ -2671,7 +2671,12 @@ extern "C" int hpf_pic_force_vjp(hpf_ctx* c, const float* pos, const float* char
         c->d_spec_phi, c->d_spec, Mc, g, c->d_box, c->d_fun, four_pi_fac, nullptr, nullptr,
         nullptr);
     HPF_LAUNCH_CHECK();
-    if ((r = exec_c2r(c, c->d_spec + Mc, c->d_grid, 3, st)) != HPF_OK) return r;
+    // (three at once where the type count has that plan: 1 and 3)
+    const int at_once = c->has_c2r[3] ? 3 : 1;
+    for (int d = 0; d < 3; d += at_once)
+        if ((r = exec_c2r(c, c->d_spec + (1 + d) * Mc, c->d_grid + (int64_t)d * M, at_once, st)) !=
+            HPF_OK)
+            return r;
     k_vjp_local<<<grid_for(n, kThreads), kThreads, 0, st>>>(c->d_grid, pos, nullptr, lam, n, 1,
                                                             M, c->d_box, grad_pos, c->d_err,
                                                             charges);
