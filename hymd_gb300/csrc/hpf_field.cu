@@ -1105,8 +1105,28 @@ int pic_chain_setup(hpf_ctx* c, cudaStream_t st) {
     return HPF_OK;
 }
 
+// Real grids off an 8-byte boundary (grids of a stack on a mesh with an odd
+// number of points): the library refuses them, so they are transformed one by
+// one, through an aligned buffer where they start on an odd float.
+bool real_misaligned(const hpf_ctx* c, const float* p) {
+    return c->fft_stage && (reinterpret_cast<uintptr_t>(p) & 7) != 0;
+}
+
 int exec_r2c(hpf_ctx* c, const float* in, float2* out, int batch, cudaStream_t st) {
     if (batch < 1 || batch > HPF_MAX_TYPES || !c->has_r2c[batch]) return HPF_ERR_ARG;
+    if (real_misaligned(c, in)) {
+        int r = HPF_OK;
+        for (int b = 0; b < batch && r == HPF_OK; ++b) {
+            const float* g = in + b * c->M;
+            if (real_misaligned(c, g)) {
+                HPF_CUDA_TRY(cudaMemcpyAsync(c->fft_stage, g, sizeof(float) * c->M,
+                                             cudaMemcpyDeviceToDevice, st));
+                g = c->fft_stage;
+            }
+            r = exec_r2c(c, g, out + b * c->Mc, 1, st);
+        }
+        return r;
+    }
     cufftHandle p = c->plan_r2c[batch];
     if (cufftSetStream(p, st) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
     if (cufftExecR2C(p, const_cast<cufftReal*>(in), reinterpret_cast<cufftComplex*>(out)) !=
@@ -1117,6 +1137,18 @@ int exec_r2c(hpf_ctx* c, const float* in, float2* out, int batch, cudaStream_t s
 
 int exec_c2r(hpf_ctx* c, const float2* in, float* out, int batch, cudaStream_t st) {
     if (batch < 1 || batch > 3 * HPF_MAX_TYPES + 1 || !c->has_c2r[batch]) return HPF_ERR_ARG;
+    if (real_misaligned(c, out)) {
+        int r = HPF_OK;
+        for (int b = 0; b < batch && r == HPF_OK; ++b) {
+            float* g = out + b * c->M;
+            const bool off = real_misaligned(c, g);
+            r = exec_c2r(c, in + b * c->Mc, off ? c->fft_stage : g, 1, st);
+            if (r == HPF_OK && off)
+                HPF_CUDA_TRY(cudaMemcpyAsync(g, c->fft_stage, sizeof(float) * c->M,
+                                             cudaMemcpyDeviceToDevice, st));
+        }
+        return r;
+    }
     cufftHandle p = c->plan_c2r[batch];
     if (cufftSetStream(p, st) != CUFFT_SUCCESS) return HPF_ERR_CUFFT;
     // cuFFT c2r may overwrite its input; all callers pass scratch spectra.
@@ -1125,7 +1157,6 @@ int exec_c2r(hpf_ctx* c, const float2* in, float* out, int batch, cudaStream_t s
         return HPF_ERR_CUFFT;
     return HPF_OK;
 }
-
 }  // namespace
 
 // ================================================================ C ABI ===
@@ -1153,6 +1184,7 @@ int hpf_ctx_destroy(hpf_ctx* c) {
     for (int b = 0; b <= 3 * HPF_MAX_TYPES + 1; ++b)
         if (c->has_c2r[b]) cufftDestroy(c->plan_c2r[b]);
     cudaFree(c->fft_work);
+    cudaFree(c->fft_stage);
     cudaFree(c->d_box);
     cudaFree(c->d_fun);
     if (c->fun_set) cudaEventDestroy(c->fun_set);
@@ -1243,6 +1275,7 @@ int hpf_ctx_create(hpf_ctx** out, int n0, int n1, int n2, int T, const double bo
         }
         c->fft_work_size = need;
         if (need) CK(cudaMalloc(&c->fft_work, need));
+        if (c->M % 2) CK(cudaMalloc(&c->fft_stage, sizeof(float) * c->M));
         for (int b = 0; b <= HPF_MAX_TYPES; ++b)
             if (c->has_r2c[b] && cufftSetWorkArea(c->plan_r2c[b], c->fft_work) != CUFFT_SUCCESS) {
                 st = HPF_ERR_CUFFT;

@@ -74,6 +74,7 @@ struct hpf_ctx {
     int* d_err;               // first device error code
     void* fft_work;
     size_t fft_work_size;
+    float* fft_stage;  // one grid, on meshes with an odd number of points
     // FP64 energy path (created on first use, outside graph capture)
     cufftHandle plan_d2z[2];  // batch T densities; T + 1 with the charges
     bool has_d2z[2];
