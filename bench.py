@@ -724,10 +724,12 @@ def run_gpu(args):
                           "host wall clock"}
 
     # ---- roofline -------------------------------------------------------------
-    # dominant kernel: the fused rRESPA inner loop.  Algorithmic bytes are
-    # those of the unfused inner step (read r, v, F; write r, v, F; bonded
-    # term data: 72 N + 16 B + 20 A + 144 D) times respa_inner; the fused
-    # kernel keeps the loop on chip, so its DRAM traffic is far lower.
+    # dominant kernel: the fused rRESPA inner loop.  Algorithmic bytes are what
+    # one launch has to move: r, v and the slow forces in, r and v out, the
+    # bonded force in and out where there is one, the bonded terms once, and
+    # with the fused paint the types (and charges) in and the 64-bit
+    # accumulators out.  The loop itself runs on chip (unfused_bytes: what
+    # respa_inner separate inner steps would move).
     peak, peak_kind = _peaks()
     T = cfg.n_types
     M = int(np.prod(cfg.mesh()))
@@ -736,13 +738,14 @@ def run_gpu(args):
     nb = topo.n_bonds if topo else 0
     na = topo.n_angles if topo else 0
     nd = topo.n_dihedrals if topo else 0
-    respa_bytes = cfg.respa_inner * (72 * n + 16 * nb + 20 * na + 144 * nd)
+    unfused_bytes = cfg.respa_inner * (72 * n + 16 * nb + 20 * na + 144 * nd)
+    n_bonded = n - (md.plan_info() or {}).get("free_beads", 0)
+    respa_bytes = (12 * n * (4 + len(md._slow_forces())) + 24 * n_bonded + 16 * nb + 20 * na
+                   + 144 * nd)
     nq = int(md.charged.numel()) if md.charged is not None else 0
     fused_paint = md._paint_fused
     if fused_paint:
-        # the launch also paints every bead (and the charged ones): the
-        # paint's contract bytes, 16 N + 4 T M (+ 16 N_q + 4 M)
-        respa_bytes += 16 * n + 4 * T * M + ((16 * nq + 4 * M) if nq else 0)
+        respa_bytes += 4 * n + 8 * T * M + ((4 * n + 8 * M) if nq else 0)
     respa_gbs = respa_bytes / (respa_ms * 1e-3) / 1e9
     traffic = _traffic(args.workload)
     # the other kernels of the step, timed stage by stage (graphs + events,
@@ -784,7 +787,9 @@ def run_gpu(args):
         info = md.plan_info() or {}
         # one warp per molecule group up to 64 beads, one CTA per group beyond
         warp = max(md.block_beads or 0, info.get("max_block_beads", 0)) <= 64
-        respa_kernel = "k_respa_warp" if warp else "k_respa_cta"
+        # (in registers up to 32 beads without four-body terms)
+        lane = warp and info.get("max_block_beads", 0) <= 32 and nd == 0
+        respa_kernel = "k_respa_lane" if lane else "k_respa_warp" if warp else "k_respa_cta"
         line = {"metric": METRIC, "value": sps * ws, "unit": "steps/s", "n_gpus": ws,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -815,10 +820,11 @@ def run_gpu(args):
                              "frac": respa_gbs / peak, "traffic": traffic.get("respa"),
                              "peak_kind": peak_kind, "ms_per_launch": respa_ms,
                              "algorithmic_bytes": respa_bytes,
-                             "bytes_basis": "respa_inner x (72 N + 16 B + 20 A + 144 D), "
-                                            "the unfused inner step's reads and writes"
-                                            + (", + the fused paint's 16 N + 4 T M (+ 16 N_q "
-                                               "+ 4 M for the charges)" if fused_paint else ""),
+                             "bytes_basis": "one fused launch: 12 N (4 + slow forces) + 24 N_bonded "
+                                            "+ 16 B + 20 A + 144 D"
+                                            + (", + the fused paint's 4 N + 8 T M (+ 4 N + 8 M "
+                                               "with charges)" if fused_paint else ""),
+                             "unfused_bytes": unfused_bytes,
                              "note": "latency-bound in practice: the loop runs on chip and "
                                      "touches DRAM once per bead per launch (traffic)"},
                 "roofline_kernels": kernels,
