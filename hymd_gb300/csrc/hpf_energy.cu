@@ -18,7 +18,7 @@
 // Accuracy: as the D2Z path's.  On deposits that are exact (beads on mesh
 // points) both are within 2 x 2^-53 of the sum of the terms' absolute values
 // of a transform in extended precision.  Two FP32 words a number would be
-// faster (380 against 502 us for a print step of 162k beads, 1353 against 1920
+// faster (369 against 502 us for a print step of 162k beads, 1353 against 1920
 // for energy and gradients of 1.3M), but hold 48 bits: 2 to 30 x 2^-53 on the
 // same deposits, a cancelling quadratic form to 2e-12 instead of 3e-15, and
 // nothing at all in units whose sums lie outside FP32's exponents.  Meshes of

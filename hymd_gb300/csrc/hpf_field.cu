@@ -284,6 +284,8 @@ struct KickDev {
 // a second one.  What bounds the gather is L1: 22 sectors a request, each
 // looked up again for the neighbour.  500k peptides (two readouts) 271 -> 264.5
 // us a step, 1.3M-bead field evaluation 371 -> 362.
+// Four blocks per SM hold it to 64 registers, which the modes with velocity
+// sums exceed: 56 to 80 bytes of spills (-Xptxas -v).
 template <int MODE, bool SCALE, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 4) k_readout(const float* __restrict__ fm, const float* __restrict__ pos,
                           const int32_t* __restrict__ types, const float* __restrict__ charges,

@@ -185,8 +185,8 @@ __global__ void k_csvr_scale_flat(float* __restrict__ v, int64_t n3,
 // per block, one block's pass over the partials and a launch of its own for
 // the scaling.  Here the pass over the partials (8 G float2 from L2) runs in
 // every block at once, with the velocities already on their way.  Whole step,
-// captured: 10k-bead melt 43.8 -> 41.0 us, 162k membrane 106.7 -> 101, 500k
-// peptides 279.5 -> 276.
+// captured: 10k-bead melt 41 -> 38 us, 162k membrane NPT 102 -> 98 and NVT
+// 97 -> 90; 500k peptides differ by less than their runs (258 to 271).
 // FLAT: one coupling group and 16-byte aligned v, as k_csvr_scale_flat.
 constexpr int kApplyAhead = 2;  // 16-byte loads in flight over the reduction
 

@@ -791,8 +791,8 @@ class RespaMD:
     def _defer_sums(self):
         """step() may leave the inner loop's sums to run beside the field
         step's first pass, which joins them.  Measured on GB300, us a step in
-        line / beside: 10k melt 42.9 / 39.2.  A barostat's box update has to
-        come before that pass.  With charges the charge chain already fills
+        line / beside: 10k melt 42 / 38, 162k membrane NVT 94 / 90.  A
+        barostat's box update has to come before that pass.  With charges the charge chain already fills
         the gap and the extra branch costs (500k peptides 273 / 287, 60k 130 /
         128, 12k 97 / 96), so there the sums stay in line; so they do in a
         subclass with a second half of its own."""
