@@ -666,7 +666,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[K], double* smem /* K*3
     }
 }
 
-// Compensated ("double-float") sum of two (hi, lo) FP32 pairs: TwoSum of the
+// Compensated ("double-float") sum of two (hi, lo) FP32 pairs: Knuth's TwoSum of the
 // high parts, then the low parts folded in and renormalised.  About 48
 // significant bits, using only the FP32 pipe.
 struct DF {
